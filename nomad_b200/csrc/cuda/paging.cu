@@ -450,6 +450,7 @@ extern "C" nomad_status nomad_paging_enable(nomad_ctx *ctx, const nomad_paging_c
   for (int w = 0; w < 2; ++w)
     if (W == 2 || w != wi) ctx->ws[w].wn = nullptr;
   ctx->scene.tri = pg->recBase;
+  ctx->scene.triCount = (int32_t)pg->recCap;
   ctx->pnodeWords = nodeRegion / 4;
   // slot words on the device (for k_publish)
   NOMAD_CUDA(ctx, pg->slots.reserve((size_t)nobj * 8 + 8));

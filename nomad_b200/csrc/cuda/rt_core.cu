@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "rt_context.h"
+#include "trace_coop.cuh"
 
 using namespace nomad_dev;
 
@@ -52,27 +53,18 @@ __device__ __forceinline__ void trace_one(const DevScene &S, const WideScene &WS
   }
 }
 
-template <int W, int STACK, bool ANY>
-__device__ __forceinline__ void trace_ray(const DevScene &S, const WideScene &WS, const float4 *__restrict__ rays,
-                                          uint64_t i, int32_t *__restrict__ hits5, uint8_t *__restrict__ occ,
-                                          uint32_t *__restrict__ counts) {
-  float4 a = __ldg(rays + 2 * i), b = __ldg(rays + 2 * i + 1);
-  RayP r = prep_ray(a, b);
-  HitRec h;
-  trace_one<W, STACK, ANY>(S, WS, r, b.w, h);
-  if (ANY) {
-    occ[i] = h.prim >= 0 ? 1 : 0;
-  } else {
-    int32_t *o = hits5 + 5 * i;
-    o[0] = h.inst;
-    o[1] = h.prim;
-    o[2] = __float_as_int(h.prim >= 0 ? h.t : INFINITY);
-    o[3] = __float_as_int(h.u);
-    o[4] = __float_as_int(h.v);
-    if (counts) warp_count_object_hit(h.prim >= 0 ? h.inst : -1, counts);
-  }
+__device__ __forceinline__ void store_result(int32_t *__restrict__ hits5, uint64_t i, const HitRec &h,
+                                             uint32_t *__restrict__ counts) {
+  int32_t *o = hits5 + 5 * i;
+  o[0] = h.inst;
+  o[1] = h.prim;
+  o[2] = __float_as_int(h.prim >= 0 ? h.t : INFINITY);
+  o[3] = __float_as_int(h.u);
+  o[4] = __float_as_int(h.v);
+  if (counts) warp_count_object_hit(h.prim >= 0 ? h.inst : -1, counts);
 }
 
+// One ray per thread (PERSIST = false) or persistent warps with cooperative leaf tests.
 template <int W, int STACK, bool ANY, bool PERSIST, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS, const float4 *__restrict__ rays,
                                                   uint64_t n, const uint32_t *__restrict__ lenDev,
@@ -80,20 +72,25 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS
                                                   int32_t *__restrict__ hits5, uint8_t *__restrict__ occ,
                                                   uint32_t *__restrict__ counts) {
   const uint64_t N = lenDev ? (uint64_t)*lenDev : n;
-  if (!PERSIST) {
+  if constexpr (!PERSIST) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) trace_ray<W, STACK, ANY>(S, WS, rays, i, hits5, occ, counts);
-    return;
-  }
-  int lane = threadIdx.x & 31;
-  for (;;) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(cursor, 32ull);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= N) break;
-    uint64_t i = base + lane;
-    if (i < N) trace_ray<W, STACK, ANY>(S, WS, rays, i, hits5, occ, counts);
-    __syncwarp();
+    if (i >= N) return;
+    float4 a = __ldg(rays + 2 * i), b = __ldg(rays + 2 * i + 1);
+    RayP r = prep_ray(a, b);
+    HitRec h;
+    trace_one<W, STACK, ANY>(S, WS, r, b.w, h);
+    if (ANY)
+      occ[i] = h.prim >= 0 ? 1 : 0;
+    else
+      store_result(hits5, i, h, counts);
+  } else {
+    __shared__ CoopShared sh;
+    coop_trace<W, STACK, ANY>(S, WS, sh, rays, (uint32_t)N, cursor, [&](uint64_t i, const HitRec &h) {
+      if (ANY)
+        occ[i] = h.prim >= 0 ? 1 : 0;
+      else
+        store_result(hits5, i, h, counts);
+    });
   }
 }
 
@@ -378,6 +375,7 @@ extern "C" nomad_status nomad_scene_upload(nomad_ctx *ctx, const float *bvh, uin
   }
   S.rootRef = L.rootRef;
   S.tlasPairs = L.tlasPairCount;
+  S.triCount = (int32_t)primCount;
   S.status = static_cast<uint32_t *>(ctx->status.p);
   ctx->primCount = primCount;
   ctx->objectCount = objectCount;
@@ -583,19 +581,28 @@ template <int W, int STACK, bool ANY, bool PERSIST, int MINB>
 nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                         unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts, cudaStream_t st) {
   auto kern = k_trace<W, STACK, ANY, PERSIST, MINB>;
-  uint64_t blocks;
-  if (PERSIST) {
-    int perSm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kBlock, 0);
-    blocks = (uint64_t)ctx->smCount * std::max(perSm, 1);
-    blocks = std::max<uint64_t>(1, std::min(blocks, (n + kBlock - 1) / kBlock));
-    NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
+  if constexpr (PERSIST) {
+    static const int perSm = [kern] {  // resident blocks per SM, of every sm_100 device
+      int k = 0;
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kBlock, 0) == cudaSuccess && k > 0 ? k : 1;
+    }();
+    // ray indices are 32 bits in the kernel; a queue's length on the device is 32 bits already
+    constexpr uint64_t kMost = 1ull << 31;
+    for (uint64_t off = 0; off < n; off += kMost) {
+      const uint64_t m = lenDev ? n : std::min(kMost, n - off);
+      const uint64_t blocks = std::min<uint64_t>((uint64_t)ctx->smCount * perSm, (m + kBlock - 1) / kBlock);
+      NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
+      kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays + 2 * off, m, lenDev, cursor,
+                                                hits5 ? hits5 + 5 * off : nullptr, occ ? occ + off : nullptr, counts);
+      NOMAD_CUDA(ctx, cudaGetLastError());
+      if (lenDev) break;
+    }
   } else {
-    blocks = (n + kBlock - 1) / kBlock;
+    const uint64_t blocks = (n + kBlock - 1) / kBlock;
     if (blocks > 0x7fffffffull) return nomad_fail(ctx, NOMAD_ERR_LIMIT, "too many rays for one call");
+    kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays, n, lenDev, cursor, hits5, occ, counts);
+    NOMAD_CUDA(ctx, cudaGetLastError());
   }
-  kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays, n, lenDev, cursor, hits5, occ, counts);
-  NOMAD_CUDA(ctx, cudaGetLastError());
   return NOMAD_OK;
 }
 
@@ -603,12 +610,17 @@ template <int W, int STACK, bool ANY, bool PERSIST>
 nomad_status launch_minb(nomad_ctx *ctx, uint32_t minBlocks, const WideScene &WS, const float4 *rays, uint64_t n,
                          const uint32_t *lenDev, unsigned long long *cursor, int32_t *hits5, uint8_t *occ,
                          uint32_t *counts, cudaStream_t st) {
-  switch (minBlocks) {
-    case 0: return launch_one<W, STACK, ANY, PERSIST, 1>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    case 10: return launch_one<W, STACK, ANY, PERSIST, 10>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    case 12: return launch_one<W, STACK, ANY, PERSIST, 12>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    case 16: return launch_one<W, STACK, ANY, PERSIST, 16>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    default: return nomad_fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "min_blocks must be 0, 10, 12 or 16");
+  if (minBlocks != 0 && minBlocks != 10 && minBlocks != 12 && minBlocks != 16)
+    return nomad_fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "min_blocks must be 0, 10, 12 or 16");
+  if constexpr (PERSIST) {  // one build, at the occupancy that was measured best
+    return launch_one<W, STACK, ANY, true, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  } else {
+    switch (minBlocks) {
+      case 0: return launch_one<W, STACK, ANY, false, 1>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+      case 10: return launch_one<W, STACK, ANY, false, 10>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+      case 12: return launch_one<W, STACK, ANY, false, 12>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+      default: return launch_one<W, STACK, ANY, false, 16>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    }
   }
 }
 

@@ -39,6 +39,7 @@ struct DevScene {
   float rmin[3], rmax[3];
   int32_t rootRef;
   uint32_t tlasPairs;
+  int32_t triCount;  // records behind tri
   uint32_t *status;
 };
 
@@ -113,26 +114,28 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
   return ax * bx + ay * by + az * bz;
 }
 
-// Tests one record; on acceptance updates h (closest) and returns true.
-// `best`/`bprim` define the current closest; for any-hit `best` is tmax and bprim INT_MIN.
-__device__ __forceinline__ bool test_prim(const DevScene &S, const RayP &r, float4 A, float4 B,
-                                          float4 C, int32_t pid, int type, HitRec &h) {
-  float tt, u = 0.0f, v = 0.0f;
+// The intersection of one record with a ray (origin o, direction d): its distance and barycentrics,
+// and whether there is one beyond kRayEps. `best` is the current closest distance; only a
+// rectangle's test uses it, to stop early.
+__device__ __forceinline__ bool intersect_prim(const DevScene &S, float ox, float oy, float oz, float dx, float dy,
+                                               float dz, float4 A, float4 B, float4 C, int32_t pid, int type,
+                                               float best, float &tt, float &u, float &v) {
+  u = v = 0.0f;
   if (type == 1) {
     // Möller–Trumbore (PathTracing.h:786-797) on v0 = A, edge1 = B, edge2 = C.
-    float hx = r.dy * C.z - r.dz * C.y;
-    float hy = r.dz * C.x - r.dx * C.z;
-    float hz = r.dx * C.y - r.dy * C.x;
+    float hx = dy * C.z - dz * C.y;
+    float hy = dz * C.x - dx * C.z;
+    float hz = dx * C.y - dy * C.x;
     float a = dot3(B.x, B.y, B.z, hx, hy, hz);
     if (!(fabsf(a) > 1e-5f)) return false;
     float f = __frcp_rn(a);
-    float sx = r.ox - A.x, sy = r.oy - A.y, sz = r.oz - A.z;
+    float sx = ox - A.x, sy = oy - A.y, sz = oz - A.z;
     u = f * dot3(sx, sy, sz, hx, hy, hz);
     if (!(u >= 0.0f && u <= 1.0f)) return false;
     float qx = sy * B.z - sz * B.y;
     float qy = sz * B.x - sx * B.z;
     float qz = sx * B.y - sy * B.x;
-    v = f * dot3(r.dx, r.dy, r.dz, qx, qy, qz);
+    v = f * dot3(dx, dy, dz, qx, qy, qz);
     if (!(v >= 0.0f && u + v <= 1.0f)) return false;
     tt = f * dot3(C.x, C.y, C.z, qx, qy, qz);
   } else if (type == 2) {
@@ -153,20 +156,20 @@ __device__ __forceinline__ bool test_prim(const DevScene &S, const RayP &r, floa
       float len = sqrtf(nl);
       nx = sn.x / len; ny = sn.y / len; nz = sn.z / len;
     }
-    float denom = dot3(nx, ny, nz, r.dx, r.dy, r.dz);
+    float denom = dot3(nx, ny, nz, dx, dy, dz);
     if (!(fabsf(denom) > 1e-5f)) return false;
-    tt = dot3(A.x - r.ox, A.y - r.oy, A.z - r.oz, nx, ny, nz) / denom;
-    if (!(tt > kRayEps && tt <= h.t)) return false;
-    float px = r.ox + tt * r.dx, py = r.oy + tt * r.dy, pz = r.oz + tt * r.dz;
+    tt = dot3(A.x - ox, A.y - oy, A.z - oz, nx, ny, nz) / denom;
+    if (!(tt > kRayEps && tt <= best)) return false;
+    float px = ox + tt * dx, py = oy + tt * dy, pz = oz + tt * dz;
     float rx = px - A.x, ry = py - A.y, rz = pz - A.z;
     float uu = dot3(rx, ry, rz, B.x, B.y, B.z) / dot3(B.x, B.y, B.z, B.x, B.y, B.z);
     float vv = dot3(rx, ry, rz, C.x, C.y, C.z) / dot3(C.x, C.y, C.z, C.x, C.y, C.z);
     if (!(fabsf(uu) <= 1.0f && fabsf(vv) <= 1.0f)) return false;
   } else if (type == 0) {
     // Sphere (PathTracing.h:751-770): center A, radius B.x; nearest root only.
-    float ocx = r.ox - A.x, ocy = r.oy - A.y, ocz = r.oz - A.z;
-    float a = dot3(r.dx, r.dy, r.dz, r.dx, r.dy, r.dz);
-    float b = dot3(ocx, ocy, ocz, r.dx, r.dy, r.dz);
+    float ocx = ox - A.x, ocy = oy - A.y, ocz = oz - A.z;
+    float a = dot3(dx, dy, dz, dx, dy, dz);
+    float b = dot3(ocx, ocy, ocz, dx, dy, dz);
     float c = dot3(ocx, ocy, ocz, ocx, ocy, ocz) - B.x * B.x;
     float disc = b * b - a * c;
     if (!(disc > 0.0f)) return false;
@@ -174,7 +177,15 @@ __device__ __forceinline__ bool test_prim(const DevScene &S, const RayP &r, floa
   } else {
     return false;
   }
-  if (!(tt > kRayEps)) return false;
+  return tt > kRayEps;
+}
+
+// Tests one record; on acceptance updates h (closest) and returns true. h.t and h.prim define the
+// current closest; for any-hit h.t is tmax and h.prim INT32_MIN.
+__device__ __forceinline__ bool test_prim(const DevScene &S, const RayP &r, float4 A, float4 B,
+                                          float4 C, int32_t pid, int type, HitRec &h) {
+  float tt, u, v;
+  if (!intersect_prim(S, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, A, B, C, pid, type, h.t, tt, u, v)) return false;
   if (!(tt < h.t || (tt == h.t && pid < h.prim))) return false;
   h.t = tt;
   h.u = u;
