@@ -2,12 +2,13 @@
 // FP32 accumulation on the tensor cores, trained on the device with AdamW. Every matrix product
 // runs on tcgen05 with tensor-memory accumulators: inference (every residency step) and the
 // training forward pass in one fused kernel (both hidden layers and the output dot product, the
-// weights staged by one bulk copy), and the backward products in a tiled GEMM kernel whose
-// operands the threads stage in the canonical shared-memory layout.
+// weights staged by one bulk copy), the backward products in two kernels whose operands arrive by
+// bulk copies of images that the kernel before laid out for them.
 //
 // The GEMMs are tiny (2,048 objects x 128 x 128 per frame; a 4,096-row training batch), so the
 // kernels are built for latency; the backward products use split-K partial sums reduced in a
-// fixed order, so training is bit-reproducible for a given seed.
+// fixed order, and bias gradients are summed row by row, so training is bit-reproducible for a
+// given seed.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -61,6 +62,8 @@ constexpr uint32_t kTcH1 = kTcW2 + 128 * kHid * 2;
 constexpr uint32_t kTcF = kTcH1 + 128 * kHid * 2;   // fp32: b1, b2, w3, b3, mean, istd
 constexpr uint32_t kTcBar = kTcF + 4 * (3 * kHid + 1 + 2 * kIn + 7);  // copy barrier, MMA barrier, TMEM slot
 constexpr size_t kTcSmem = kTcBar + 24;
+constexpr uint32_t kTcIdx = kTcBar + 24;            // training: the tile's sample indices
+constexpr size_t kTcSmemTrain = kTcIdx + 4 * kTcRows;
 constexpr uint32_t kStatusWaitExpired = 1u << 1;
 constexpr long long kTcWaitPolls = 1ll << 22;
 
@@ -122,20 +125,45 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
 // them whenever the weights change), so one bulk asynchronous copy stages both.
 // FEAT: the rows are the residency step's objects; each thread computes its object's features
 // (nomad_res::object_features, the same code as the feature kernel) instead of reading X.
-// SAVE (training): also stores what the backward pass needs, row-major: the standardised inputs
-// (bf16, n x 32), Z1 = X W1^T + b1 (fp32), H1 = ReLU(Z1) (bf16) and Z2 = H1 W2^T + b2 (fp32).
-struct FwdSave {
-  __nv_bfloat16 *xbf, *h1;
-  float *z1, *z2;
+// TRAIN: the rows are a batch, row r the sample perm[(cursor + r) % n] (or r itself without perm);
+// besides the outputs' errors the kernel stores what the backward pass needs, per 128-row tile:
+//   ximg, h1img, z2img  X, H1 and dZ2 as operand images (canon_off). One image serves both as a
+//          K-major operand (rows against columns: dH1) and, rows being the K of the weight
+//          gradients, as an MN-major one (dW1, dW2), so nothing is transposed.
+//   g2c, g3c  dZ2 and ReLU(Z2) dy column by column (fp32, col_off), whose row-ordered sums are db2
+//          and dw3; mask: Z1 > 0, 128 bits a row.
+struct TrainBufs {
+  unsigned char *ximg, *h1img, *z2img, *z1img;
+  float *g1c, *g2c, *g3c, *dy, *se;
+  uint32_t *mask;
+  float *part1, *part2;
 };
+struct TrainRows {
+  const float *T;
+  const uint32_t *perm;
+  uint64_t cursor, n;
+};
+constexpr uint32_t kTileBytes = 128 * kHid * 2;    // a 128-row tile of 128 columns
+constexpr uint32_t kXTileBytes = 128 * kInPad * 2;  // and of X
 
-template <bool FEAT, bool SAVE>
+// Float offset of (column c, row r) in the fp32 columns: tiles of 128 rows, a column's 128 rows
+// together, their 16-byte groups permuted by the column so that 32 lanes reading the same group of
+// 32 columns meet different banks.
+__device__ __forceinline__ size_t col_off(int c, int r) {
+  return (size_t)(r >> 7) * (128 * kHid) + c * 128 + (((((r & 127) >> 2) ^ (c & 31)) << 2) | (r & 3));
+}
+
+__device__ __forceinline__ void bulk_store(void *dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+
+template <bool FEAT, bool TRAIN>
 __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict__ X, uint64_t n,
                                                         const float *__restrict__ P,
                                                         const unsigned char *__restrict__ Wc, float *__restrict__ y,
                                                         uint32_t *__restrict__ status, nomad_res::FeatArgs fa,
-                                                        FwdSave sv) {
-  extern __shared__ __align__(16) unsigned char smem[];
+                                                        TrainRows rows, TrainBufs tb) {
+  extern __shared__ __align__(1024) unsigned char smem[];
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
   float *sB1 = reinterpret_cast<float *>(smem + kTcF);
   float *sB2 = sB1 + kHid;
@@ -182,6 +210,17 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict_
   }
   __syncthreads();
   const uint64_t row0 = (uint64_t)blockIdx.x * kTcRows;
+  uint32_t *sIdx = reinterpret_cast<uint32_t *>(smem + kTcIdx);  // TRAIN: the tile's samples
+  float target = 0.0f;
+  if constexpr (TRAIN) {
+    uint32_t s = 0;
+    if (row0 + tid < n) {
+      s = rows.perm ? rows.perm[(rows.cursor + row0 + tid) % rows.n] : (uint32_t)(row0 + tid);
+      target = rows.T[s];
+    }
+    sIdx[tid] = s;
+    __syncthreads();
+  }
   if constexpr (FEAT) {
     float f[NOMAD_FEATURES];
     const bool live = row0 + tid < n;
@@ -192,13 +231,14 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict_
       *reinterpret_cast<__nv_bfloat16 *>(smem + kTcX + canon_off(tid, k)) = __float2bfloat16_rn(v);
     }
   } else {
-    for (int i = tid; i < kTcRows * kInPad; i += 128) {
+#pragma unroll
+    for (int i0 = 0; i0 < kTcRows * kInPad; i0 += 128) {  // all of a thread's loads in flight at once
+      const int i = i0 + tid;
       const int r = i / kInPad, f = i % kInPad;
       float v = 0.0f;
-      if (f < kIn && row0 + r < n) v = (X[(row0 + r) * kIn + f] - sMean[f]) * sIstd[f];
+      if (f < kIn && row0 + r < n) v = (X[(TRAIN ? (uint64_t)sIdx[r] : row0 + r) * kIn + f] - sMean[f]) * sIstd[f];
       const __nv_bfloat16 b = __float2bfloat16_rn(v);
       *reinterpret_cast<__nv_bfloat16 *>(smem + kTcX + canon_off(r, f)) = b;
-      if (SAVE && row0 + r < n) sv.xbf[(row0 + r) * kInPad + f] = b;
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -222,28 +262,36 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict_
   // epilogue 1: bias, ReLU, BF16 into the layer-2 operand (row = this thread's lane)
   const int r = tid;
   const bool rowLive = row0 + r < n;
-#pragma unroll
+  // The 32-column steps of the epilogues stay loops: unrolled, each instruction runs once per
+  // block, and fetching 100 KB of code took longer (45 us a training launch) than the work.
+#pragma unroll 1
   for (int c0 = 0; c0 < kHid; c0 += 32) {
     float v[32];
     tc_ld32(lane_base + c0, v);
+    uint32_t mask = 0u;
+    uint32_t h[16];
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
       const float za = v[j] + sB1[c0 + j], zb = v[j + 1] + sB1[c0 + j + 1];
-      const uint32_t h = pack_bf16(fmaxf(za, 0.0f), fmaxf(zb, 0.0f));
-      *reinterpret_cast<uint32_t *>(smem + kTcH1 + canon_off(r, c0 + j)) = h;
-      if (SAVE && rowLive) {
-        const uint64_t o = (row0 + r) * kHid + c0 + j;
-        sv.z1[o] = za;
-        sv.z1[o + 1] = zb;
-        *reinterpret_cast<uint32_t *>(sv.h1 + o) = h;
-      }
+      h[j / 2] = pack_bf16(fmaxf(za, 0.0f), fmaxf(zb, 0.0f));
+      if (TRAIN) mask |= (za > 0.0f ? 1u << j : 0u) | (zb > 0.0f ? 2u << j : 0u);
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4 *>(smem + kTcH1 + canon_off(r, c0 + 8 * q)) =
+          make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+    if (TRAIN && rowLive) tb.mask[(row0 + r) * 4 + c0 / 32] = mask;
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   // layer 2: D2 = H1 . W2^T, K = 128 in eight steps
+  if (TRAIN && tid == 0) {  // the operand images of X and H1 go out while it runs
+    bulk_store(tb.ximg + (uint64_t)blockIdx.x * kXTileBytes, sbase + kTcX, kXTileBytes);
+    bulk_store(tb.h1img + (uint64_t)blockIdx.x * kTileBytes, sbase + kTcH1, kTileBytes);
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
   if (tid == 0) {
 #pragma unroll
     for (int s = 0; s < kHid / 16; ++s)
@@ -255,18 +303,50 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict_
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   // epilogue 2: ReLU(D2 + b2) . w3 + b3 for this thread's row
   float acc = 0.0f;
-#pragma unroll
+#pragma unroll 1
   for (int c0 = 0; c0 < kHid; c0 += 32) {
     float v[32];
     tc_ld32(lane_base + 128 + c0, v);
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       const float z = v[j] + sB2[c0 + j];
-      if (SAVE && rowLive) sv.z2[(row0 + r) * kHid + c0 + j] = z;
       acc += fmaxf(z, 0.0f) * sW3[c0 + j];
     }
   }
-  if (row0 + r < n) y[row0 + r] = ok ? acc + sB3[0] : 0.0f;
+  if constexpr (TRAIN) {
+    // the error of this row, its output gradient 2 (y - t) / n, and dZ2 = dy w3 (Z2 > 0)
+    const float d = (ok ? acc + sB3[0] : 0.0f) - target;
+    const float dy = 2.0f * d / (float)(int)n;
+    if (rowLive) {
+      tb.dy[row0 + r] = dy;
+      tb.se[row0 + r] = d * d;
+    }
+    unsigned char *img = tb.z2img + (uint64_t)blockIdx.x * kTileBytes;
+#pragma unroll 1
+    for (int c0 = 0; c0 < kHid; c0 += 32) {
+      float v[32];
+      tc_ld32(lane_base + 128 + c0, v);
+      uint32_t h[16];
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float za = v[j] + sB2[c0 + j], zb = v[j + 1] + sB2[c0 + j + 1];
+        const float ga = za > 0.0f ? dy * sW3[c0 + j] : 0.0f, gb = zb > 0.0f ? dy * sW3[c0 + j + 1] : 0.0f;
+        const size_t oa = col_off(c0 + j, (int)row0 + r), ob = col_off(c0 + j + 1, (int)row0 + r);
+        tb.g2c[oa] = ga;
+        tb.g2c[ob] = gb;
+        tb.g3c[oa] = (za > 0.0f ? za : 0.0f) * dy;
+        tb.g3c[ob] = (zb > 0.0f ? zb : 0.0f) * dy;
+        h[j / 2] = rowLive ? pack_bf16(ga, gb) : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4 *>(img + canon_off(r, c0 + 8 * q)) =
+            make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+    }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  } else {
+    if (row0 + r < n) y[row0 + r] = ok ? acc + sB3[0] : 0.0f;
+  }
   if (!ok && tid == 0) atomicOr(status, kStatusWaitExpired);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -276,36 +356,19 @@ __global__ void __launch_bounds__(128) k_mlp_forward_tc(const float *__restrict_
   }
 }
 
-// ---- backward GEMMs on the 5th-generation tensor cores (tcgen05) ---------------------------
-// C[z][M][N] (fp32) = sum over split z's K range of op(A)[M][K] op(B)[K][N], where A is stored
-// [M][K] (TA = 0) or [K][M] (TA = 1) and B [K][N] (TB = 0) or [N][K] (TB = 1), all bf16. One CTA
-// of 128 threads owns a 128-row tile of C and all NT (= N rounded up: 32 or 128) columns,
-// accumulated in tensor memory. K advances 64 at a time: the threads stage the A tile (128 x 64)
-// and the B tile (NT x 64) in shared memory in the canonical K-major layout (whatever the global
-// layout, so transposed operands cost nothing extra), then one thread issues four
-// tcgen05.mma (M = 128, N = NT, K = 16) and commits to an mbarrier that every thread waits on
-// before the tiles are overwritten. Elements past M, N or the split's K range are staged as zero.
-// Split-K partial tiles are summed afterwards in a fixed order (k_reduce_splits), so a gradient
-// is bit-reproducible.
-constexpr int kGemmK = 64;
-
-// Byte offset of element (r, k) of an R-row K-major operand tile in the canonical layout.
-template <int R>
-__device__ __forceinline__ uint32_t canon_off_r(int r, int k) {
-  return (uint32_t)((((k >> 3) * (R / 8) + (r >> 3)) << 7) + ((r & 7) << 4) + ((k & 7) << 1));
+// ---- backward pass on the 5th-generation tensor cores (tcgen05) -----------------------------
+// Descriptor of an operand image read with its rows as K (MN-major): 8 x 8 core matrices, the next
+// eight rows 128 B on (leading offset), the next eight columns 2,048 B on (stride offset).
+__device__ __forceinline__ uint64_t rows_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3fffu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(2048u >> 4) << 32) |
+         (1ull << 46);
 }
 
-// Descriptor of an R-row operand: next K chunk (R / 8) * 128 B away, next row group 128 B away.
-template <int R>
-__device__ __forceinline__ uint64_t canon_desc_r(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3fffu) | ((uint64_t)((R / 8 * 128) >> 4) << 16) |
-         ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
-}
-
+// D[128][NT] += A B with both operands MN-major.
 template <int NT>
-__device__ __forceinline__ void tc_mma_n(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-  // kind::f16: FP32 accumulator, BF16 A and B, both K-major, N = NT, M = 128
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);
+__device__ __forceinline__ void tc_mma_rows(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(NT >> 3) << 17) |
+                             ((128u >> 4) << 24);
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
@@ -313,202 +376,347 @@ __device__ __forceinline__ void tc_mma_n(uint32_t dtmem, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
-template <bool TA, bool TB, int NT>
-__global__ void __launch_bounds__(128) k_gemm_tc(const __nv_bfloat16 *__restrict__ A,
-                                                 const __nv_bfloat16 *__restrict__ B, float *__restrict__ C,
-                                                 int M, int N, int K, int lda, int ldb, int kPerSplit,
-                                                 uint32_t *__restrict__ status) {
-  static_assert(NT == 32 || NT == 64 || NT == 128, "tile width");
-  __shared__ __align__(1024) unsigned char sA[128 * kGemmK * 2];
-  __shared__ __align__(1024) unsigned char sB[NT * kGemmK * 2];
-  __shared__ __align__(8) unsigned long long sBar;
-  __shared__ uint32_t sTmem;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t aBase = static_cast<uint32_t>(__cvta_generic_to_shared(sA));
-  const uint32_t bBase = static_cast<uint32_t>(__cvta_generic_to_shared(sB));
-  const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(&sBar));
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+__device__ __forceinline__ void bar_init(uint32_t bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// One bulk copy (no multicast) of this GPU's own memory.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+      "r"(bytes), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// Tensor memory of the block (cols columns) and its barriers, before and after the products.
+__device__ __forceinline__ uint32_t tc_begin(uint32_t slot, const uint32_t *slotPtr, uint32_t bar0, int bars, uint32_t cols) {
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < bars; ++i) bar_init(bar0 + 8 * i);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     static_cast<uint32_t>(__cvta_generic_to_shared(&sTmem))),
-                 "r"((uint32_t)NT)
-                 : "memory");
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = sTmem;
-  const int m0 = blockIdx.y * 128;
-  const int kBeg = blockIdx.z * kPerSplit, kEnd = min(K, kBeg + kPerSplit);
-  const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f);
-  uint32_t phase = 0;
-  bool ok = true, issued = false;
-  for (int k0 = kBeg; k0 < kEnd && ok; k0 += kGemmK) {
-    for (int i = tid; i < 128 * kGemmK; i += 128) {
-      // consecutive threads read consecutive addresses of the stored layout
-      const int r = TA ? i % 128 : i / kGemmK, c = TA ? i / 128 : i % kGemmK;
-      const int m = m0 + r, k = k0 + c;
-      __nv_bfloat16 v = zero;
-      if (m < M && k < kEnd) v = TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-      *reinterpret_cast<__nv_bfloat16 *>(sA + canon_off_r<128>(r, c)) = v;
-    }
-    for (int i = tid; i < NT * kGemmK; i += 128) {
-      const int r = TB ? i / kGemmK : i % NT, c = TB ? i % kGemmK : i / NT;
-      const int k = k0 + c;
-      __nv_bfloat16 v = zero;
-      if (r < N && k < kEnd) v = TB ? B[(size_t)r * ldb + k] : B[(size_t)k * ldb + r];
-      *reinterpret_cast<__nv_bfloat16 *>(sB + canon_off_r<NT>(r, c)) = v;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0) {
-#pragma unroll
-      for (int s = 0; s < kGemmK / 16; ++s)
-        tc_mma_n<NT>(tmem, canon_desc_r<128>(aBase + s * 2 * (128 / 8 * 128)),
-                     canon_desc_r<NT>(bBase + s * 2 * (NT / 8 * 128)), (k0 > kBeg || s > 0) ? 1u : 0u);
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                   : "memory");
-    }
-    issued = true;
-    ok = __syncthreads_and(tc_wait(bar, phase) ? 1 : 0) != 0;  // one outcome for the whole CTA
-    phase ^= 1u;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  }
-  if (!ok) {
-    // the last commit did not arrive in time: give the MMAs in flight one more bounded wait
-    // before the tensor memory is released, and report it
-    tc_wait(bar, phase ^ 1u);
-    if (tid == 0) atomicOr(status, kStatusWaitExpired);
-  }
-  const int row = m0 + tid;
-  float *Cz = C + (size_t)blockIdx.z * M * N;
-  const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-  for (int c0 = 0; c0 < NT; c0 += 32) {
-    float v[32];
-    if (issued) {
-      tc_ld32(lane_base + c0, v);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = 0.0f;  // empty K range
-    }
-    if (row < M) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (c0 + j < N) Cz[(size_t)row * N + c0 + j] = ok ? v[j] : 0.0f;
-    }
-  }
+  return *slotPtr;
+}
+__device__ __forceinline__ void tc_end(uint32_t tmem, uint32_t cols) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)NT) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
   }
 }
 
-// Sums split-K partials in fixed order: out[i] = sum_z part[z][i].
-__global__ void k_reduce_splits(const float *__restrict__ part, int splits, size_t count,
-                                float *__restrict__ out) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(size_t)z * count + i];
-    out[i] = s;
+// One split of a weight gradient: D[128][NT] = sum of A^T B over the 64-row blocks [b0, b0 + nb) of two
+// images (A 128 columns, B NT columns), 16 rows an instruction. One thread runs a ring of kRing
+// tiles of bulk copies ahead of the MMAs; the others wait for the last commit. The partial goes
+// out row-major.
+constexpr int kRing = 3;
+template <int NT>
+__device__ __forceinline__ void split_product(unsigned char *smem, const unsigned char *A, const unsigned char *B, int b0,
+                                              int nb, float *__restrict__ out, uint32_t *__restrict__ status) {
+  constexpr uint32_t bBytes = NT * 128 * 2, stage = kTileBytes + bBytes;
+  const int tid = threadIdx.x;
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t bars = base + kRing * stage;  // full[kRing], free[kRing], done
+  const uint32_t fin = bars + 16 * kRing;
+  uint32_t *slot = reinterpret_cast<uint32_t *>(smem + kRing * stage + 16 * kRing + 8);
+  const uint32_t tmem = tc_begin(fin + 8, slot, bars, 2 * kRing + 1, NT);
+  if (tid == 0) {
+    const int t0 = b0 / 2, nt = (b0 + nb - 1) / 2 - t0 + 1;
+    auto load = [&](int i) {
+      const uint32_t s = base + (i % kRing) * stage, bar = bars + 8 * (i % kRing);
+      bar_expect(bar, stage);
+      bulk_load(s, A + (size_t)(t0 + i) * kTileBytes, kTileBytes, bar);
+      bulk_load(s + kTileBytes, B + (size_t)(t0 + i) * bBytes, bBytes, bar);
+    };
+    int loaded = 0;
+    for (; loaded < kRing && loaded < nt; ++loaded) load(loaded);
+    bool ok = true, first = true;
+    for (int i = 0; i < nt && ok; ++i) {
+      const uint32_t s = base + (i % kRing) * stage;
+      ok = tc_wait(bars + 8 * (i % kRing), (i / kRing) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // the split may begin or end in the middle of a tile
+      const int k0 = max(0, (b0 - 2 * (t0 + i)) * 4), k1 = min(8, (b0 + nb - 2 * (t0 + i)) * 4);
+      for (int k = k0; k < k1; ++k) {
+        tc_mma_rows<NT>(tmem, rows_desc(s + k * 256), rows_desc(s + kTileBytes + k * 256), first ? 0u : 1u);
+        first = false;
+      }
+      if (loaded < nt) {  // refill this stage once its products are done
+        tc_commit(bars + 8 * (kRing + i % kRing));
+        ok = tc_wait(bars + 8 * (kRing + i % kRing), (i / kRing) & 1) && ok;
+        if (ok) load(loaded++);
+      }
+    }
+    // a wait that ran out: let the copies in flight land before the block ends
+    if (!ok)
+      for (int i = max(0, loaded - kRing); i < loaded; ++i) tc_wait(bars + 8 * (i % kRing), (i / kRing) & 1);
+    tc_commit(fin);
+    if (!ok) atomicOr(status, kStatusWaitExpired);
+  }
+  const bool ok = __syncthreads_and(tc_wait(fin, 0) ? 1 : 0) != 0;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!ok && tid == 0) atomicOr(status, kStatusWaitExpired);
+  const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) * 32) << 16);
+  float4 *row = reinterpret_cast<float4 *>(out + (size_t)tid * NT);
+#pragma unroll 1
+  for (int c0 = 0; c0 < NT; c0 += 32) {
+    float v[32];
+    tc_ld32(lane_base + c0, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) row[c0 / 4 + j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+  tc_end(tmem, NT);
+}
+constexpr size_t split_smem(int nt) { return kRing * (kTileBytes + (size_t)nt * 256) + 16 * kRing + 16; }
+
+// The hidden layers' backward products. Blocks [0, tiles): dH1 = dZ2 W2 of one 128-row tile and
+// dZ1 = dH1 (Z1 > 0), stored as a bf16 operand image and as fp32 columns. Blocks from tiles on: one
+// split of dW2 = dZ2^T H1.
+__global__ void __launch_bounds__(128) k_train_hidden(int n, int tiles, int blocksPerSplit,
+                                                      const unsigned char *__restrict__ W2t, TrainBufs tb,
+                                                      uint32_t *__restrict__ status) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x >= tiles) {
+    const int z = blockIdx.x - tiles, b0 = z * blocksPerSplit;
+    split_product<kHid>(smem, tb.z2img, tb.h1img, b0, min(blocksPerSplit, n / 64 - b0),
+                        tb.part2 + (size_t)z * kHid * kHid, status);
+    return;
+  }
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t bar = base + 2 * kTileBytes, fin = bar + 8;
+  const uint32_t tmem = tc_begin(fin + 8, reinterpret_cast<uint32_t *>(smem + 2 * kTileBytes + 16), bar, 2, kHid);
+  if (tid == 0) {
+    bar_expect(bar, 2 * kTileBytes);
+    bulk_load(base, tb.z2img + (size_t)blockIdx.x * kTileBytes, kTileBytes, bar);
+    bulk_load(base + kTileBytes, W2t, kTileBytes, bar);
+  }
+  bool ok = tc_wait(bar, 0);
+  if (tid == 0) {
+#pragma unroll
+    for (int s = 0; s < kHid / 16; ++s)
+      tc_mma(tmem, canon_desc(base + s * 2 * 2048), canon_desc(base + kTileBytes + s * 2 * 2048), s > 0);
+    tc_commit(fin);
+  }
+  ok = tc_wait(fin, 0) && ok;
+  if (!ok) {
+    tc_wait(bar, 0);
+    atomicOr(status, kStatusWaitExpired);
+  }
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t lane_base = tmem + ((uint32_t)((tid >> 5) * 32) << 16);
+  const int r = blockIdx.x * kTcRows + tid;
+  const bool live = r < n;
+  unsigned char *img = tb.z1img + (size_t)blockIdx.x * kTileBytes;
+#pragma unroll 1
+  for (int c0 = 0; c0 < kHid; c0 += 32) {
+    float v[32];
+    tc_ld32(lane_base + c0, v);
+    const uint32_t mask = live ? tb.mask[(size_t)r * 4 + c0 / 32] : 0u;
+    uint32_t h[16];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float ga = (mask >> j) & 1u ? v[j] : 0.0f, gb = (mask >> (j + 1)) & 1u ? v[j + 1] : 0.0f;
+      h[j / 2] = pack_bf16(ga, gb);
+      tb.g1c[col_off(c0 + j, r)] = ga;
+      tb.g1c[col_off(c0 + j + 1, r)] = gb;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4 *>(img + canon_off(tid, c0 + 8 * q)) =
+          make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+  }
+  tc_end(tmem, kHid);
+}
+constexpr size_t kHiddenSmem = std::max<size_t>(split_smem(kHid), 2 * kTileBytes + 32);
+
+// Row-ordered column sums: out[c] = sum over rows r, in order, of col[c][r], 32 columns (from c0, laid
+// out by col_off) a block and a lane a column, or of one plain column (PLAIN). The chain of
+// dependent additions sets the time (4 cycles a row: 8.7 us for 4,096 rows at 1.9 GHz), so one warp
+// does nothing but wait, load four rows at a time from shared memory and add, while another
+// thread keeps a ring of bulk copies (128 rows each) ahead of it.
+constexpr int kSumRing = 8;
+constexpr uint32_t kSumStage = 32 * 128 * 4;
+template <bool PLAIN>
+__device__ __forceinline__ void ordered_sums(unsigned char *smem, int n, int c0, const float *__restrict__ col,
+                                             float *__restrict__ out, uint32_t *__restrict__ status) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem)), bars = base + kSumRing * kSumStage;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2 * kSumRing; ++i) bar_init(bars + 8 * i);  // full, free
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  const int tiles = (n + 127) / 128;
+  bool ok = true;
+  if (warp == 1 && lane == 0) {
+    for (int t = 0; t < tiles; ++t) {
+      const int s = t % kSumRing;
+      if (t >= kSumRing && !tc_wait(bars + 8 * (kSumRing + s), (t / kSumRing - 1) & 1)) {
+        ok = false;
+        break;
+      }
+      const uint32_t bytes = PLAIN ? min(128, n - t * 128) * 4 : kSumStage;
+      bar_expect(bars + 8 * s, bytes);
+      bulk_load(base + s * kSumStage, col + (PLAIN ? (size_t)t * 128 : (size_t)t * (128 * kHid) + c0 * 128), bytes,
+                bars + 8 * s);
+    }
+  } else if (warp == 0) {
+    // chunks of 32 rows, the next one loading while one is added
+    float sum = 0.0f;
+    const int chunks = n / 32, x = PLAIN ? 0 : lane;  // n is a multiple of 64: an even number
+    float4 p[8], q[8];
+    auto at = [&](int i) {
+      return reinterpret_cast<const float4 *>(smem + (size_t)((i >> 2) % kSumRing) * kSumStage) + (PLAIN ? 0 : lane * 32);
+    };
+    // one load between every four additions: the loads fill the chain's idle issue slots
+    auto step = [&](const float4 (&v)[8], float4 (&w)[8], const float4 *src, int g) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        w[k] = src[(g + k) ^ x];
+        sum += v[k].x;
+        sum += v[k].y;
+        sum += v[k].z;
+        sum += v[k].w;
+      }
+    };
+    ok = __all_sync(0xffffffffu, tc_wait(bars, 0));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = at(0)[k ^ x];
+#pragma unroll 1
+    for (int i = 0; i < chunks && ok; i += 2) {
+      step(p, q, at(i), ((i + 1) & 3) * 8);
+      int next = i + 2;
+      if (next < chunks) {
+        if ((next & 3) == 0) {  // the tile is in registers: free it, wait for the next
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 8 * (kSumRing + (i >> 2) % kSumRing))
+                         : "memory");
+          const int t = next >> 2;
+          ok = __all_sync(0xffffffffu, tc_wait(bars + 8 * (t % kSumRing), (t / kSumRing) & 1));
+        }
+      } else {
+        next = i;  // nothing follows: what is loaded is not used
+      }
+      step(q, p, at(next), (next & 3) * 8);
+    }
+    if (!PLAIN || lane == 0) out[lane] = sum;
+  }
+  if (!ok && lane == 0) {
+    // a wait that ran out: let the copies in flight land before the block ends
+    for (int s = 0; s < kSumRing; ++s) tc_wait(bars + 8 * s, 0);
+    atomicOr(status, kStatusWaitExpired);
+  }
+  __syncthreads();
+}
+
+// The input layer's weight gradient and the vectors' gradients. Blocks [0, splits): one split of
+// dW1 = dZ1^T X. Then four blocks of 32 columns each for db1 = sum dZ1, db2 = sum dZ2 and
+// dw3 = sum ReLU(Z2) dy, and one for db3 = sum dy.
+__global__ void __launch_bounds__(128) k_train_input(int n, int splits, int blocksPerSplit, float *__restrict__ G,
+                                                     TrainBufs tb, uint32_t *__restrict__ status) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  if ((int)blockIdx.x < splits) {
+    const int z = blockIdx.x, b0 = z * blocksPerSplit;
+    split_product<kInPad>(smem, tb.z1img, tb.ximg, b0, min(blocksPerSplit, n / 64 - b0),
+                          tb.part1 + (size_t)z * kHid * kInPad, status);
+    return;
+  }
+  const int q = blockIdx.x - splits, c0 = (q & 3) * 32;
+  if (q < 12) {
+    const float *col = q < 4 ? tb.g1c : q < 8 ? tb.g2c : tb.g3c;
+    ordered_sums<false>(smem, n, c0, col, G + (q < 4 ? oB1 : q < 8 ? oB2 : oW3) + c0, status);
+  } else {
+    ordered_sums<true>(smem, n, 0, tb.dy, G + oB3, status);
+  }
+}
+constexpr size_t kInputSmem = std::max<size_t>(split_smem(kInPad), kSumRing * kSumStage + 16 * kSumRing);
+
+// The bf16 weights of the tensor-core kernels: W1 then W2 in the canonical operand layout (one
+// block), and W2 transposed for dH1. W1's padded input columns stay zero.
+__device__ __forceinline__ void store_weight(int i, float p, unsigned char *__restrict__ Wc, unsigned char *__restrict__ W2t) {
+  if (i < oB1) {
+    const int c = i % kInPad;
+    *reinterpret_cast<__nv_bfloat16 *>(Wc + canon_off(i / kInPad, c)) = __float2bfloat16_rn(c < kIn ? p : 0.0f);
+  } else if (i >= oW2 && i < oB2) {
+    const int r = (i - oW2) / kHid, c = (i - oW2) % kHid;
+    const __nv_bfloat16 w = __float2bfloat16_rn(p);
+    *reinterpret_cast<__nv_bfloat16 *>(Wc + (kTcW2 - kTcW1) + canon_off(r, c)) = w;
+    *reinterpret_cast<__nv_bfloat16 *>(W2t + canon_off(c, r)) = w;
   }
 }
 
-// dy = 2 (y - t) / B; per-row squared errors for the loss.
-__global__ void k_mse_grad(const float *__restrict__ y, const float *__restrict__ t, int B,
-                           float *__restrict__ dy, float *__restrict__ se) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < B) {
-    float d = y[i] - t[i];
-    dy[i] = 2.0f * d / (float)B;
-    se[i] = d * d;
+// Completes the gradient (split-K partials summed in split order) and, with update, takes the AdamW
+// step over the trainable part of the blob (everything before the feature statistics) and
+// refreshes the bf16 weights. Without update the gradient goes to G.
+__global__ void __launch_bounds__(128) k_adamw(float *__restrict__ P, float *__restrict__ G, float *__restrict__ m,
+                                               float *__restrict__ v, int splits, TrainBufs tb, bool update, float lr,
+                                               float b1, float b2, float eps, float wd, float bc1, float bc2,
+                                               unsigned char *__restrict__ Wc, unsigned char *__restrict__ W2t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= oMean) return;
+  const bool w1 = i < oB1, w2 = i >= oW2 && i < oB2;
+  float g;
+  if (w1 || w2) {
+    const size_t count = w1 ? kHid * kInPad : kHid * kHid;
+    const float *part = w1 ? tb.part1 + i : tb.part2 + (i - oW2);
+    g = 0.0f;
+#pragma unroll 8
+    for (int z = 0; z < splits; ++z) g += part[(size_t)z * count];
+  } else {
+    g = G[i];
   }
+  if (!update) {
+    G[i] = g;
+    return;
+  }
+  const float mi = b1 * m[i] + (1.0f - b1) * g;
+  const float vi = b2 * v[i] + (1.0f - b2) * g * g;
+  m[i] = mi;
+  v[i] = vi;
+  const float mh = mi / bc1, vh = vi / bc2;
+  float p = P[i];
+  if (w1 || w2 || (i >= oW3 && i < oB3)) p = p - lr * wd * p;
+  p = p - lr * mh / (sqrtf(vh) + eps);
+  P[i] = p;
+  store_weight(i, p, Wc, W2t);
 }
 
-// dZ2 = dy * w3 * (Z2 > 0) (bf16 for the GEMMs, fp32 kept for the bias gradient).
-__global__ void k_dz2(const float *__restrict__ dy, const float *__restrict__ z2, const float *__restrict__ P,
-                      int B, __nv_bfloat16 *__restrict__ dz2b, float *__restrict__ dz2f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < B * kHid) {
-    int r = i / kHid, c = i % kHid;
-    float v = z2[i] > 0.0f ? dy[r] * P[oW3 + c] : 0.0f;
-    dz2f[i] = v;
-    dz2b[i] = __float2bfloat16_rn(v);
-  }
+__global__ void k_refresh_bf16(const float *__restrict__ P, unsigned char *__restrict__ Wc,
+                               unsigned char *__restrict__ W2t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < oMean) store_weight(i, P[i], Wc, W2t);
 }
 
-// dZ1 = dH1 * (Z1 > 0).
-__global__ void k_dz1(const float *__restrict__ dh1, const float *__restrict__ z1, int B,
-                      __nv_bfloat16 *__restrict__ dz1b, float *__restrict__ dz1f) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < B * kHid) {
-    float v = z1[i] > 0.0f ? dh1[i] : 0.0f;
-    dz1f[i] = v;
-    dz1b[i] = __float2bfloat16_rn(v);
+// Mean squared error of each step's batch, the rows added in order in double.
+__global__ void __launch_bounds__(128) k_loss(const float *__restrict__ se, int n, float *__restrict__ loss) {
+  __shared__ float tile[2048];
+  const float *row = se + (size_t)blockIdx.x * n;
+  double acc = 0.0;
+  for (int r0 = 0; r0 < n; r0 += 2048) {
+    const int m = min(2048, n - r0);
+    for (int i = threadIdx.x; i < m; i += 128) tile[i] = row[r0 + i];
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int i = 0; i < m; ++i) acc += tile[i];
+    __syncthreads();
   }
-}
-
-// Column sums in fixed row order: out[c] = sum_r M[r][c] * (w ? w[r] : 1); one thread per column.
-__global__ void k_colsum(const float *__restrict__ M, const float *__restrict__ w, int rows, int cols,
-                         float *__restrict__ out) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < cols) {
-    float s = 0.0f;
-    for (int r = 0; r < rows; ++r) s += M[(size_t)r * cols + c] * (w ? w[r] : 1.0f);
-    out[c] = s;
-  }
-}
-
-// AdamW over the trainable part of the blob (everything before the feature statistics).
-__global__ void k_adamw(float *__restrict__ P, const float *__restrict__ G, float *__restrict__ m,
-                        float *__restrict__ v, int count, float lr, float b1, float b2, float eps,
-                        float wd, float bc1, float bc2) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) {
-    float g = G[i];
-    float mi = b1 * m[i] + (1.0f - b1) * g;
-    float vi = b2 * v[i] + (1.0f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float mh = mi / bc1, vh = vi / bc2;
-    bool isWeight = (i < oB1) || (i >= oW2 && i < oB2) || (i >= oW3 && i < oB3);
-    float p = P[i];
-    if (isWeight) p = p - lr * wd * p;
-    P[i] = p - lr * mh / (sqrtf(vh) + eps);
-  }
-}
-
-// bf16 copies of W1 and W2 (W1's padded input columns stay zero), row-major for the training
-// kernels and packed in the canonical layout of the tcgen05 inference kernel (W1 then W2).
-__global__ void k_refresh_bf16(const float *__restrict__ P, __nv_bfloat16 *__restrict__ W1b,
-                               __nv_bfloat16 *__restrict__ W2b, unsigned char *__restrict__ Wc) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kHid * kInPad) {
-    const __nv_bfloat16 w = __float2bfloat16_rn((i % kInPad) < kIn ? P[oW1 + i] : 0.0f);
-    W1b[i] = w;
-    *reinterpret_cast<__nv_bfloat16 *>(Wc + canon_off(i / kInPad, i % kInPad)) = w;
-  }
-  if (i < kHid * kHid) {
-    const __nv_bfloat16 w = __float2bfloat16_rn(P[oW2 + i]);
-    W2b[i] = w;
-    *reinterpret_cast<__nv_bfloat16 *>(Wc + (kTcW2 - kTcW1) + canon_off(i / kHid, i % kHid)) = w;
-  }
-}
-
-// Gathers a mini-batch of raw features and targets.
-__global__ void k_gather(const float *__restrict__ X, const float *__restrict__ T, const uint32_t *__restrict__ idx,
-                         int B, float *__restrict__ xb, float *__restrict__ tb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < B * kIn) xb[i] = X[(size_t)idx[i / kIn] * kIn + i % kIn];
-  if (i < B) tb[i] = T[idx[i]];
+  if (threadIdx.x == 0) loss[blockIdx.x] = (float)(acc / n);
 }
 
 }  // namespace
@@ -517,10 +725,8 @@ __global__ void k_gather(const float *__restrict__ X, const float *__restrict__ 
 
 struct MlpState {
   bool ready = false;
-  DeviceBuf P, W1b, W2b, Wc, M, V, G;
-  DeviceBuf X, T, idx, xb, tb, y, z1, h1, z2, xbf, dy, se, dz2b, dz2f, dh1, dz1b, dz1f, part;
-  uint64_t trainCap = 0;
-  int batchCap = 0;
+  DeviceBuf P, Wc, W2t, M, V, G;
+  DeviceBuf X, T, perm[2], ximg, h1img, z2img, z1img, g1c, g2c, g3c, dy, se, mask, part1, part2, loss;
   DeviceBuf inX, inY;
 };
 
@@ -532,17 +738,15 @@ MlpState &mlp(nomad_ctx *ctx) {
 }
 
 nomad_status refresh(nomad_ctx *ctx, MlpState &S) {
-  int n = kHid * kHid;
-  k_refresh_bf16<<<(n + 255) / 256, 256, 0, ctx->stream>>>(S.P.as<const float>(), S.W1b.as<__nv_bfloat16>(),
-                                                            S.W2b.as<__nv_bfloat16>(), S.Wc.as<unsigned char>());
+  k_refresh_bf16<<<(oMean + 255) / 256, 256, 0, ctx->stream>>>(S.P.as<const float>(), S.Wc.as<unsigned char>(),
+                                                               S.W2t.as<unsigned char>());
   NOMAD_CUDA(ctx, cudaGetLastError());
   return NOMAD_OK;
 }
 
 nomad_status ensure(nomad_ctx *ctx, MlpState &S) {
   NOMAD_CUDA(ctx, S.P.reserve(kParams * 4));
-  NOMAD_CUDA(ctx, S.W1b.reserve(kHid * kInPad * 2));
-  NOMAD_CUDA(ctx, S.W2b.reserve(kHid * kHid * 2));
+  NOMAD_CUDA(ctx, S.W2t.reserve(kTileBytes));
   NOMAD_CUDA(ctx, S.Wc.reserve(kTcWBytes));
   NOMAD_CUDA(ctx, S.M.reserve(kParams * 4));
   NOMAD_CUDA(ctx, S.V.reserve(kParams * 4));
@@ -554,7 +758,9 @@ nomad_status ensure(nomad_ctx *ctx, MlpState &S) {
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_mlp_forward_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kTcSmem));
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_mlp_forward_tc<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTcSmem));
+                                         (int)kTcSmemTrain));
+    NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_train_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHiddenSmem));
+    NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_train_input, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInputSmem));
     attr = true;
   }
   return NOMAD_OK;
@@ -572,7 +778,7 @@ nomad_status nomad_mlp_infer_device(nomad_ctx *ctx, const float *X, uint64_t n, 
   k_mlp_forward_tc<false, false><<<blocks, 128, kTcSmem, ctx->stream>>>(X, n, S.P.as<const float>(),
                                                                         S.Wc.as<const unsigned char>(), y,
                                                                         ctx->status.as<uint32_t>(),
-                                                                        nomad_res::FeatArgs{}, FwdSave{});
+                                                                        nomad_res::FeatArgs{}, TrainRows{}, TrainBufs{});
   NOMAD_CUDA(ctx, cudaGetLastError());
   return NOMAD_OK;
 }
@@ -584,7 +790,7 @@ nomad_status nomad_mlp_score_objects(nomad_ctx *ctx, const nomad_res::FeatArgs *
   const unsigned blocks = (fa->n + kTcRows - 1) / kTcRows;
   k_mlp_forward_tc<true, false><<<blocks, 128, kTcSmem, ctx->stream>>>(nullptr, fa->n, S.P.as<const float>(),
                                                                        S.Wc.as<const unsigned char>(), keys,
-                                                                       ctx->status.as<uint32_t>(), *fa, FwdSave{});
+                                                                       ctx->status.as<uint32_t>(), *fa, TrainRows{}, TrainBufs{});
   NOMAD_CUDA(ctx, cudaGetLastError());
   return NOMAD_OK;
 }
@@ -755,87 +961,58 @@ extern "C" nomad_status nomad_mlp_infer(nomad_ctx *ctx, const float *features, u
 
 namespace {
 
-nomad_status ensure_batch(nomad_ctx *ctx, MlpState &S, int B, int splits) {
-  if (S.batchCap < B) {
-    NOMAD_CUDA(ctx, S.idx.reserve((size_t)B * 4));
-    NOMAD_CUDA(ctx, S.xb.reserve((size_t)B * kIn * 4));
-    NOMAD_CUDA(ctx, S.tb.reserve((size_t)B * 4));
-    NOMAD_CUDA(ctx, S.y.reserve((size_t)B * 4));
-    NOMAD_CUDA(ctx, S.z1.reserve((size_t)B * kHid * 4));
-    NOMAD_CUDA(ctx, S.h1.reserve((size_t)B * kHid * 2));
-    NOMAD_CUDA(ctx, S.z2.reserve((size_t)B * kHid * 4));
-    NOMAD_CUDA(ctx, S.xbf.reserve((size_t)B * kInPad * 2));
-    NOMAD_CUDA(ctx, S.dy.reserve((size_t)B * 4));
-    NOMAD_CUDA(ctx, S.se.reserve((size_t)B * 4));
-    NOMAD_CUDA(ctx, S.dz2b.reserve((size_t)B * kHid * 2));
-    NOMAD_CUDA(ctx, S.dz2f.reserve((size_t)B * kHid * 4));
-    NOMAD_CUDA(ctx, S.dh1.reserve((size_t)B * kHid * 4));
-    NOMAD_CUDA(ctx, S.dz1b.reserve((size_t)B * kHid * 2));
-    NOMAD_CUDA(ctx, S.dz1f.reserve((size_t)B * kHid * 4));
-    S.batchCap = B;
-  }
-  NOMAD_CUDA(ctx, S.part.reserve((size_t)std::max(splits, 1) * kHid * kHid * 4));
+// Split-K of the weight gradients: a split takes a whole number of 64-row blocks.
+struct Splits {
+  int blocks, count;
+};
+Splits batch_splits(int B) {
+  const int want = std::max(1, std::min(32, B / 256));
+  const int per = (B / want + 63) / 64;
+  return {per, (B / 64 + per - 1) / per};
+}
+
+nomad_status ensure_batch(nomad_ctx *ctx, MlpState &S, int B, uint64_t losses) {
+  const size_t tiles = ((size_t)B + 127) / 128, splits = batch_splits(B).count;
+  NOMAD_CUDA(ctx, S.ximg.reserve(tiles * kXTileBytes));
+  for (DeviceBuf *b : {&S.h1img, &S.z2img, &S.z1img}) NOMAD_CUDA(ctx, b->reserve(tiles * kTileBytes));
+  for (DeviceBuf *b : {&S.g1c, &S.g2c, &S.g3c}) NOMAD_CUDA(ctx, b->reserve(tiles * 128 * kHid * 4));
+  NOMAD_CUDA(ctx, S.dy.reserve((size_t)B * 4));
+  NOMAD_CUDA(ctx, S.se.reserve((size_t)B * 4 * losses));
+  NOMAD_CUDA(ctx, S.loss.reserve(4 * losses));
+  NOMAD_CUDA(ctx, S.mask.reserve((size_t)B * 16));
+  NOMAD_CUDA(ctx, S.part1.reserve(splits * kHid * kInPad * 4));
+  NOMAD_CUDA(ctx, S.part2.reserve(splits * kHid * kHid * 4));
   return NOMAD_OK;
 }
 
-int batch_splits(int B) { return std::max(1, std::min(32, B / 256)); }
-
-// Forward and backward of the batch in S.xb / S.tb (B rows, B a multiple of 64): the gradient of
-// the mean squared error with respect to every trainable parameter into S.G (the blob's layout;
-// W1's padded input columns get 0), the per-row squared errors into S.se. Mixed precision as in
-// the forward pass: BF16 operands of every product (standardised inputs, weights, hidden
-// activations, the gradients that flow into a product), FP32 accumulation, FP32 biases and
-// output layer; split-K partial sums reduced in a fixed order.
-nomad_status batch_gradient(nomad_ctx *ctx, MlpState &S, int B) {
+// Forward and backward of a batch of B samples of X and rows.T (B a multiple of 64): the gradient
+// of the mean squared error with respect to every trainable parameter, as split-K partials and in
+// S.G (k_adamw completes it; W1's padded input columns get 0), the per-row squared errors into se.
+// Mixed precision as in the forward pass: BF16 operands of every product (standardised inputs,
+// weights, hidden activations, the gradients that flow into a product), FP32 accumulation, FP32
+// biases and output layer.
+//
+// Three launches a step and one for the update: a step of 4,096 rows takes 48 us (forward 19,
+// hidden 7, input 17, update 4). It took 757 us as 17 launches whose column sums added 4,096 rows
+// straight from memory, a thread a column, three times about 200 us. The chain of those additions is
+// what bounds a step now (17.2k cycles of dependent additions): their order is the result's, so the
+// sums of both layers run side by side, after the one that ends last.
+nomad_status batch_gradient(nomad_ctx *ctx, MlpState &S, int B, const float *X, const TrainRows &rows, float *se,
+                            TrainBufs &tb) {
   cudaStream_t s = ctx->stream;
-  const int splits = batch_splits(B);
-  float *Pm = S.P.as<float>(), *G = S.G.as<float>();
+  const Splits sp = batch_splits(B);
+  const int tiles = (B + kTcRows - 1) / kTcRows;
   uint32_t *status = ctx->status.as<uint32_t>();
-  k_mlp_forward_tc<false, true><<<(B + kTcRows - 1) / kTcRows, 128, kTcSmem, s>>>(
-      S.xb.as<const float>(), B, Pm, S.Wc.as<const unsigned char>(), S.y.as<float>(), status, nomad_res::FeatArgs{},
-      FwdSave{S.xbf.as<__nv_bfloat16>(), S.h1.as<__nv_bfloat16>(), S.z1.as<float>(), S.z2.as<float>()});
-  k_mse_grad<<<(B + 255) / 256, 256, 0, s>>>(S.y.as<const float>(), S.tb.as<const float>(), B, S.dy.as<float>(),
-                                             S.se.as<float>());
-  k_dz2<<<(B * kHid + 255) / 256, 256, 0, s>>>(S.dy.as<const float>(), S.z2.as<const float>(), Pm, B,
-                                               S.dz2b.as<__nv_bfloat16>(), S.dz2f.as<float>());
-  // dw3[c] = sum_r relu(z2[r][c]) * dy[r]; db3 = sum_r dy[r]
-  {
-    // relu(z2) into dh1, which is free until dH1 below (z2 itself feeds dz2 above)
-    float *h2 = S.dh1.as<float>();
-    size_t cnt = (size_t)B * kHid;
-    k_dz1<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(S.z2.as<const float>(), S.z2.as<const float>(), B,
-                                                       S.dz1b.as<__nv_bfloat16>(), h2);
-    k_colsum<<<1, kHid, 0, s>>>(h2, S.dy.as<const float>(), B, kHid, G + oW3);
-    k_colsum<<<1, 1, 0, s>>>(S.dy.as<const float>(), nullptr, B, 1, G + oB3);
-  }
-  k_colsum<<<1, kHid, 0, s>>>(S.dz2f.as<const float>(), nullptr, B, kHid, G + oB2);
-  // dW2[n][k] = sum_i dZ2[i][n] H1[i][k]: A = dZ2^T (stored [B][128]), B = H1 [B][128]
-  {
-    int kPer = ((B / splits) + kGemmK - 1) / kGemmK * kGemmK;
-    int sp = (B + kPer - 1) / kPer;
-    dim3 grid(1, 1, sp);
-    k_gemm_tc<true, false, kHid><<<grid, 128, 0, s>>>(S.dz2b.as<const __nv_bfloat16>(), S.h1.as<const __nv_bfloat16>(),
-                                                      S.part.as<float>(), kHid, kHid, B, kHid, kHid, kPer, status);
-    k_reduce_splits<<<64, 256, 0, s>>>(S.part.as<const float>(), sp, (size_t)kHid * kHid, G + oW2);
-  }
-  // dH1[i][k] = sum_n dZ2[i][n] W2[n][k]: A = dZ2 [B][128], B = W2 [128(n)][128(k)] row-major = [K][N]
-  {
-    dim3 grid(1, (B + 127) / 128, 1);
-    k_gemm_tc<false, false, kHid><<<grid, 128, 0, s>>>(S.dz2b.as<const __nv_bfloat16>(), S.W2b.as<const __nv_bfloat16>(),
-                                                       S.dh1.as<float>(), B, kHid, kHid, kHid, kHid, kHid, status);
-  }
-  k_dz1<<<(B * kHid + 255) / 256, 256, 0, s>>>(S.dh1.as<const float>(), S.z1.as<const float>(), B,
-                                               S.dz1b.as<__nv_bfloat16>(), S.dz1f.as<float>());
-  k_colsum<<<1, kHid, 0, s>>>(S.dz1f.as<const float>(), nullptr, B, kHid, G + oB1);
-  // dW1[n][k] = sum_i dZ1[i][n] X[i][k]: A = dZ1^T, B = Xbf [B][32]
-  {
-    int kPer = ((B / splits) + kGemmK - 1) / kGemmK * kGemmK;
-    int sp = (B + kPer - 1) / kPer;
-    dim3 grid(1, 1, sp);
-    k_gemm_tc<true, false, kInPad><<<grid, 128, 0, s>>>(S.dz1b.as<const __nv_bfloat16>(), S.xbf.as<const __nv_bfloat16>(),
-                                                        S.part.as<float>(), kHid, kInPad, B, kHid, kInPad, kPer, status);
-    k_reduce_splits<<<16, 256, 0, s>>>(S.part.as<const float>(), sp, (size_t)kHid * kInPad, G + oW1);
-  }
+  tb = TrainBufs{S.ximg.as<unsigned char>(), S.h1img.as<unsigned char>(), S.z2img.as<unsigned char>(),
+                 S.z1img.as<unsigned char>(), S.g1c.as<float>(), S.g2c.as<float>(), S.g3c.as<float>(),
+                 S.dy.as<float>(), se,
+                 S.mask.as<uint32_t>(), S.part1.as<float>(), S.part2.as<float>()};
+  k_mlp_forward_tc<false, true><<<tiles, 128, kTcSmemTrain, s>>>(X, B, S.P.as<const float>(),
+                                                                 S.Wc.as<const unsigned char>(), nullptr, status,
+                                                                 nomad_res::FeatArgs{}, rows, tb);
+  k_train_hidden<<<tiles + sp.count, 128, kHiddenSmem, s>>>(B, tiles, sp.blocks, S.W2t.as<const unsigned char>(), tb,
+                                                            status);
+  k_train_input<<<sp.count + 13, 128, kInputSmem, s>>>(B, sp.count, sp.blocks, S.G.as<float>(), tb, status);
   NOMAD_CUDA(ctx, cudaGetLastError());
   return NOMAD_OK;
 }
@@ -855,11 +1032,12 @@ extern "C" nomad_status nomad_mlp_train(nomad_ctx *ctx, const float *features, c
     if (st != NOMAD_OK) return st;
   }
   cudaStream_t s = ctx->stream;
-  // Feature statistics (double accumulation on the host), stored in the blob.
-  std::vector<double> mean(kIn, 0.0), sq(kIn, 0.0);
+  // Feature statistics (double accumulation on the host, each feature in sample order), stored in
+  // the blob.
+  double mean[kIn] = {}, sq[kIn] = {};
   for (uint64_t i = 0; i < n; ++i)
     for (int f = 0; f < kIn; ++f) {
-      double v = features[i * kIn + f];
+      const double v = features[i * kIn + f];
       mean[f] += v;
       sq[f] += v * v;
     }
@@ -876,49 +1054,70 @@ extern "C" nomad_status nomad_mlp_train(nomad_ctx *ctx, const float *features, c
   NOMAD_CUDA(ctx, cudaMemsetAsync(S.M.p, 0, kParams * 4, s));
   NOMAD_CUDA(ctx, cudaMemsetAsync(S.V.p, 0, kParams * 4, s));
   const int B = (int)batch;
-  if (S.trainCap < n) {
-    NOMAD_CUDA(ctx, S.X.reserve(n * kIn * 4));
-    NOMAD_CUDA(ctx, S.T.reserve(n * 4));
-    S.trainCap = n;
+  // The squared errors of up to this many steps wait on the device for k_loss (at most 64 MB).
+  const uint32_t keep = loss_out ? std::max(1u, std::min<uint32_t>(steps, (16u << 20) / batch)) : 1u;
+  NOMAD_CUDA(ctx, S.X.reserve(n * kIn * 4));
+  NOMAD_CUDA(ctx, S.T.reserve(n * 4));
+  for (auto &p : S.perm) NOMAD_CUDA(ctx, p.reserve(n * 4));
+  {
+    nomad_status st = ensure_batch(ctx, S, B, keep);
+    if (st != NOMAD_OK) return st;
   }
   NOMAD_CUDA(ctx, cudaMemcpyAsync(S.X.p, features, n * kIn * 4, cudaMemcpyHostToDevice, s));
   NOMAD_CUDA(ctx, cudaMemcpyAsync(S.T.p, targets, n * 4, cudaMemcpyHostToDevice, s));
-  {
-    nomad_status st = ensure_batch(ctx, S, B, batch_splits(B));
-    if (st != NOMAD_OK) return st;
-  }
+  // Each epoch's permutation goes up on a copy stream into one of two buffers, so the host shuffles
+  // and sends the next one while the steps of this one run. used[k]: the steps that read buffer k;
+  // sent: the copy the next steps wait for.
+  struct Events {
+    cudaEvent_t used[2] = {nullptr, nullptr}, sent = nullptr;
+    cudaStream_t copy = nullptr, compute = nullptr;
+    ~Events() {  // also after an error: nothing of this call may still be in flight
+      cudaStreamSynchronize(copy);
+      cudaStreamSynchronize(compute);
+      for (cudaEvent_t e : {used[0], used[1], sent})
+        if (e) cudaEventDestroy(e);
+    }
+  };
   std::mt19937_64 rng(seed ^ 0x5EEDull);
   std::vector<uint32_t> perm(n);
   std::iota(perm.begin(), perm.end(), 0u);
+  Events ev;
+  ev.copy = ctx->copyStreams[0];
+  ev.compute = s;
+  for (cudaEvent_t *e : {&ev.used[0], &ev.used[1], &ev.sent})
+    NOMAD_CUDA(ctx, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   uint64_t cursor = n;
-  std::vector<float> se(B);
+  int buf = 1;
+  bool first = true;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  float *Pm = S.P.as<float>(), *G = S.G.as<float>();
   for (uint32_t step = 0; step < steps; ++step) {
     if (cursor + B > n) {
       std::shuffle(perm.begin(), perm.end(), rng);
+      if (!first) NOMAD_CUDA(ctx, cudaEventRecord(ev.used[buf], s));
+      first = false;
+      buf ^= 1;
+      NOMAD_CUDA(ctx, cudaStreamWaitEvent(ev.copy, ev.used[buf], 0));
+      NOMAD_CUDA(ctx, cudaMemcpyAsync(S.perm[buf].p, perm.data(), n * 4, cudaMemcpyHostToDevice, ev.copy));
+      NOMAD_CUDA(ctx, cudaEventRecord(ev.sent, ev.copy));
+      NOMAD_CUDA(ctx, cudaStreamWaitEvent(s, ev.sent, 0));
       cursor = 0;
     }
-    std::vector<uint32_t> bidx(B);
-    for (int i = 0; i < B; ++i) bidx[i] = perm[(cursor + i) % n];
+    TrainBufs tb;
+    float *se = S.se.as<float>() + (size_t)(loss_out ? step % keep : 0) * B;
+    nomad_status st = batch_gradient(ctx, S, B, S.X.as<const float>(),
+                                     TrainRows{S.T.as<const float>(), S.perm[buf].as<const uint32_t>(), cursor, n}, se, tb);
+    if (st != NOMAD_OK) return st;
     cursor += B;
-    NOMAD_CUDA(ctx, cudaMemcpyAsync(S.idx.p, bidx.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s));
-    k_gather<<<(B * kIn + 255) / 256, 256, 0, s>>>(S.X.as<const float>(), S.T.as<const float>(),
-                                                   S.idx.as<const uint32_t>(), B, S.xb.as<float>(), S.tb.as<float>());
-    nomad_status st = batch_gradient(ctx, S, B);
-    if (st != NOMAD_OK) return st;
-    float bc1 = 1.0f - std::pow(b1, (float)(step + 1)), bc2 = 1.0f - std::pow(b2, (float)(step + 1));
-    k_adamw<<<(oMean + 255) / 256, 256, 0, s>>>(Pm, G, S.M.as<float>(), S.V.as<float>(), oMean, lr, b1, b2, eps, wd,
-                                                bc1, bc2);
-    st = refresh(ctx, S);
-    if (st != NOMAD_OK) return st;
+    const float bc1 = 1.0f - std::pow(b1, (float)(step + 1)), bc2 = 1.0f - std::pow(b2, (float)(step + 1));
+    k_adamw<<<(oMean + 127) / 128, 128, 0, s>>>(S.P.as<float>(), S.G.as<float>(), S.M.as<float>(), S.V.as<float>(),
+                                                batch_splits(B).count, tb, true, lr, b1, b2, eps, wd, bc1, bc2,
+                                                S.Wc.as<unsigned char>(), S.W2t.as<unsigned char>());
     NOMAD_CUDA(ctx, cudaGetLastError());
-    if (loss_out) {
-      NOMAD_CUDA(ctx, cudaMemcpyAsync(se.data(), S.se.p, (size_t)B * 4, cudaMemcpyDeviceToHost, s));
-      NOMAD_CUDA(ctx, cudaStreamSynchronize(s));
-      double acc = 0.0;
-      for (int i = 0; i < B; ++i) acc += se[i];
-      loss_out[step] = (float)(acc / B);
+    if (loss_out && (step + 1 == steps || (step + 1) % keep == 0)) {
+      const uint32_t done = step % keep + 1;
+      k_loss<<<done, 128, 0, s>>>(S.se.as<const float>(), B, S.loss.as<float>());
+      NOMAD_CUDA(ctx, cudaGetLastError());
+      NOMAD_CUDA(ctx, cudaMemcpyAsync(loss_out + (step + 1 - done), S.loss.p, (size_t)done * 4, cudaMemcpyDeviceToHost, s));
     }
   }
   NOMAD_CUDA(ctx, cudaStreamSynchronize(s));
@@ -934,14 +1133,21 @@ extern "C" nomad_status nomad_mlp_gradient(nomad_ctx *ctx, const float *features
   MlpState &S = mlp(ctx);
   if (!S.ready) return nomad_fail(ctx, NOMAD_ERR_NOT_READY, "MLP not initialised or trained");
   const int B = (int)n;
-  nomad_status st = ensure_batch(ctx, S, B, batch_splits(B));
+  nomad_status st = ensure_batch(ctx, S, B, 1);
   if (st != NOMAD_OK) return st;
   cudaStream_t s = ctx->stream;
-  NOMAD_CUDA(ctx, cudaMemcpyAsync(S.xb.p, features, n * kIn * 4, cudaMemcpyHostToDevice, s));
-  NOMAD_CUDA(ctx, cudaMemcpyAsync(S.tb.p, targets, n * 4, cudaMemcpyHostToDevice, s));
+  NOMAD_CUDA(ctx, S.X.reserve(n * kIn * 4));
+  NOMAD_CUDA(ctx, S.T.reserve(n * 4));
+  NOMAD_CUDA(ctx, cudaMemcpyAsync(S.X.p, features, n * kIn * 4, cudaMemcpyHostToDevice, s));
+  NOMAD_CUDA(ctx, cudaMemcpyAsync(S.T.p, targets, n * 4, cudaMemcpyHostToDevice, s));
   NOMAD_CUDA(ctx, cudaMemsetAsync(S.G.p, 0, kParams * 4, s));
-  st = batch_gradient(ctx, S, B);
+  TrainBufs tb;
+  st = batch_gradient(ctx, S, B, S.X.as<const float>(), TrainRows{S.T.as<const float>(), nullptr, 0, n}, S.se.as<float>(),
+                      tb);
   if (st != NOMAD_OK) return st;
+  k_adamw<<<(oMean + 127) / 128, 128, 0, s>>>(S.P.as<float>(), S.G.as<float>(), nullptr, nullptr, batch_splits(B).count,
+                                              tb, false, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 1.0f, nullptr, nullptr);
+  NOMAD_CUDA(ctx, cudaGetLastError());
   NOMAD_CUDA(ctx, cudaMemcpyAsync(grad, S.G.p, kParams * 4, cudaMemcpyDeviceToHost, s));
   std::vector<float> se(B);
   NOMAD_CUDA(ctx, cudaMemcpyAsync(se.data(), S.se.p, (size_t)B * 4, cudaMemcpyDeviceToHost, s));
