@@ -145,7 +145,9 @@ typedef struct nomad_tune_result {
 nomad_status nomad_autotune(nomad_ctx *ctx, const nomad_ray *rays, uint64_t n, uint32_t repeats,
                             uint32_t flags, nomad_tune_result *out);
 
-/* Chooses the traversal variant used by the trace calls (NOMAD_KERNEL_*). */
+/* Chooses the traversal variant used by the trace calls (NOMAD_KERNEL_*). Until one is chosen, and
+ * with NOMAD_KERNEL_AUTO, the library picks per scene (nomad_get_traversal then reports the binary
+ * per-thread walk) and calls on one context may overlap on several streams. */
 nomad_status nomad_set_kernel(nomad_ctx *ctx, uint32_t kernel);
 
 /* Full traversal configuration (no counterpart in the reference, which has one kernel). The

@@ -837,7 +837,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
     int cur = 0;
     for (uint32_t depth = 0; depth < maxDepth; ++depth) {
       k_bounce_reset<<<1, 1, 0, s>>>(C, cur);
-      nomad_status rs = nomad_trace_variant(ctx, ctx->trav, false, F.qRays[cur].as<const float4>(), P, &C->qlen[kQ * (cur)],
+      nomad_status rs = nomad_trace_queue(ctx, false, F.qRays[cur].as<const float4>(), P, &C->qlen[kQ * (cur)],
                                             &C->cursor[0], F.hits.as<int32_t>(), nullptr, nullptr, s);
       if (rs != NOMAD_OK) return rs;
       if (objHits && ctx->res.testsOn) {  // per-object "rays tested" for the hit posterior
@@ -856,7 +856,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
                                          F.thr.as<float4>(), F.rad.as<float4>(), ctx->shadeRec.as<const float4>(),
                                          ctx->matTable.as<const float4>(), L, C, cur, objHits, plan.on ? 1 : 0,
                                          primHits);
-      rs = nomad_trace_variant(ctx, ctx->trav, true, F.sRays.as<const float4>(), P, &C->qlen[kQ * (2)], &C->cursor[1],
+      rs = nomad_trace_queue(ctx, true, F.sRays.as<const float4>(), P, &C->qlen[kQ * (2)], &C->cursor[1],
                                nullptr, F.sOcc.as<uint8_t>(), nullptr, s);
       if (rs != NOMAD_OK) return rs;
       k_resolve<<<gridPT, kPtBlock, 0, s>>>(F.sIds.as<const uint32_t>(), F.sContrib.as<const float4>(),
@@ -886,6 +886,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
     key_put(key, ctx->res.tlas.p);
     key_put(key, dOut);
     key_put(key, ctx->trav);
+    key_put(key, ctx->travAuto);
     key_put(key, ctx->scene);
     for (const WideScene &w : ctx->ws) {
       key_put(key, w.wn);
@@ -1756,7 +1757,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
                                                ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, sCur, F.refMask.as<uint32_t>(), ra,
                                                F.refRays.as<float4>(), F.refIds.as<uint32_t>(), C);
     NOMAD_CUDA(ctx, cudaGetLastError());
-    nomad_status ts = nomad_trace_variant(ctx, ctx->trav, true, F.refRays.as<const float4>(), P * cf.candidates,
+    nomad_status ts = nomad_trace_queue(ctx, true, F.refRays.as<const float4>(), P * cf.candidates,
                                           &C->qlen[kQ * (3)], &C->cursor[1], nullptr, F.refOcc.as<uint8_t>(), nullptr, s);
     if (ts != NOMAD_OK) return ts;
     k_restir_ref_vis<<<grid, kPtBlock, 0, s>>>(F.refIds.as<const uint32_t>(), F.refOcc.as<const uint8_t>(),
@@ -1768,7 +1769,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
                                                 F.refContrib.as<float4>(), F.reuseMask.as<uint32_t>(),
                                                 F.refRays.as<float4>(), F.refIds.as<uint32_t>(), C);
     NOMAD_CUDA(ctx, cudaGetLastError());
-    ts = nomad_trace_variant(ctx, ctx->trav, true, F.refRays.as<const float4>(), P * kRefReuse, &C->qlen[kQ * (3)],
+    ts = nomad_trace_queue(ctx, true, F.refRays.as<const float4>(), P * kRefReuse, &C->qlen[kQ * (3)],
                              &C->cursor[1], nullptr, F.refOcc.as<uint8_t>(), nullptr, s);
     if (ts != NOMAD_OK) return ts;
     k_restir_ref_vis5<<<grid, kPtBlock, 0, s>>>(F.refIds.as<const uint32_t>(), F.refOcc.as<const uint8_t>(),

@@ -122,11 +122,12 @@ __device__ __forceinline__ bool intersect_tri(float4 o, float4 d, float4 A, floa
   return (fabsf(a) > 1e-5f) & (u >= 0.0f) & (u <= 1.0f) & (v >= 0.0f) & (u + v <= 1.0f) & (tt > kRayEps);
 }
 
-// Walks the rays of the batch (N < 2^32); DONE(i, h) stores the result of ray i (called by the lanes
+// Walks the rays of the batch (N < 2^32): the warp's own share of `chunk` rays, or, with a cursor, 32
+// rays at a time from it; DONE(i, h) stores the result of ray i (called by the lanes
 // that finished one, warp-divergent).
 template <int W, int STACK, bool ANY, typename DONE>
 __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &WS, CoopShared &sh,
-                                           const float4 *__restrict__ rays, uint32_t N,
+                                           const float4 *__restrict__ rays, uint32_t N, uint32_t chunk,
                                            unsigned long long *__restrict__ cursor, DONE done) {
   const int tid = threadIdx.x, lane = tid & 31, wb = tid & ~31;
   const unsigned lt = (1u << lane) - 1u;
@@ -139,8 +140,13 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
   int32_t ref = kEmptyRef;
   uint32_t ray = kNoRay;  // the lane's ray, until its result is stored
   bool more = true, mixed = false;
-  if (lane == 0) sh.left[wb >> 5] = 0;
+  if (lane == 0) {
+    const uint64_t first = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (wb >> 5)) * chunk;
+    sh.next[wb >> 5] = (uint32_t)first;
+    sh.left[wb >> 5] = cursor || first >= N ? 0u : min(chunk, N - (uint32_t)first);
+  }
   __syncwarp();
+  if (!cursor && sh.left[wb >> 5] == 0) return;
   for (;;) {
     while (ref == kEmptyRef && sp > 0) {  // the newest entry that still starts before the bound
       const int2 e = stk[--sp];
@@ -189,9 +195,11 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
       if (!more) break;  // nothing busy and nothing left
       uint32_t next = sh.next[wb >> 5], left = sh.left[wb >> 5];
       if (left == 0) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(cursor, 32ull);
-        base = __shfl_sync(kFull, base, 0);
+        unsigned long long base = N;
+        if (cursor) {
+          if (lane == 0) base = atomicAdd(cursor, 32ull);
+          base = __shfl_sync(kFull, base, 0);
+        }
         if (base >= N) {
           more = false;
           continue;

@@ -599,6 +599,7 @@ extern "C" nomad_status nomad_set_traversal(nomad_ctx *ctx, const nomad_traversa
   std::string why;
   if (!nomad_traversal_ok(ctx, *cfg, &why)) return nomad_fail(ctx, NOMAD_ERR_UNSUPPORTED, why);
   ctx->trav = *cfg;
+  ctx->travAuto = false;
   if (!ctx->trav.block) ctx->trav.block = 128;
   return NOMAD_OK;
 }
@@ -711,6 +712,7 @@ extern "C" nomad_status nomad_autotune_sweep(nomad_ctx *ctx, const nomad_ray *ra
   cudaEventDestroy(e1);
   if (rc != NOMAD_OK) return rc;
   ctx->trav = bestCfg;
+  ctx->travAuto = false;
   if (count) *count = measured;
   if (best) *best = bestCfg;
   return NOMAD_OK;

@@ -102,3 +102,32 @@ def test_odd_rays(nb, ctx, small_city, kernel):
     ctx.set_kernel(kernel)
     assert np.array_equal(_bits(ctx.trace_closest(rays)), _bits(want))
     assert np.array_equal(ctx.trace_any(rays), occ)
+
+
+@pytest.mark.parametrize("n", [1, 1000, 150_001, 700_003])
+def test_unchosen_kernel(nb, small_city, n):
+    """A context that never chose a kernel returns the per-thread binary walk's hits, also when two
+    of its calls overlap on two streams, and still reports that walk's configuration."""
+    import torch
+
+    sb = small_city[1]
+    base = raysets.aimed_rays(sb, min(n, 50_000), 5)
+    rays = torch.from_numpy(np.tile(base, -(-n // base.shape[0]))[:n].view(np.float32).reshape(-1, 8)).cuda()
+    c = nb.Context(0)
+    try:
+        c.upload(sb)
+        assert c.traversal()["width"] == 2 and c.traversal()["persistent"] == 0
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        outs = [torch.zeros((n, 5), dtype=torch.int32, device="cuda") for _ in range(3)]
+        torch.cuda.synchronize()
+        for s, o in zip(streams, outs):
+            c.set_stream(s.cuda_stream)
+            c.trace_closest_dev(rays.data_ptr(), n, o.data_ptr())
+        torch.cuda.synchronize()
+        c.set_stream(0)
+        c.set_kernel(1)
+        c.trace_closest_dev(rays.data_ptr(), n, outs[2].data_ptr())
+        c.sync()
+        assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[2])
+    finally:
+        c.close()
