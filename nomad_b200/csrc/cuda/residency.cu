@@ -359,6 +359,7 @@ __device__ void lights_rebuild(const uint4 *__restrict__ em, uint32_t ne, const 
   for (uint32_t k = threadIdx.x; k < c; k += blockDim.x) {
     const float prev = k > 0 ? cdf[k - 1] : 0.0f;
     nomad_pt::light_record(prims, mats, idx[k], cdf[k] - prev, total, rec + 5ull * k);
+    nomad_pt::light_cull(prims, idx[k], rec + 5ull * ne + 2ull * k);  // behind the records
   }
 }
 
@@ -651,7 +652,7 @@ nomad_status nomad_residency_init(nomad_ctx *ctx) {
   NOMAD_CUDA(ctx, cudaMemcpy(R.emit.p, emit.data(), (size_t)N * 4, cudaMemcpyHostToDevice));
   FrameState &F = ctx->frame;
   NOMAD_CUDA(ctx, F.lightIdx.reserve(std::max<size_t>(1, em.size()) * 4));
-  NOMAD_CUDA(ctx, F.lightRec.reserve(std::max<size_t>(1, em.size()) * 80));
+  NOMAD_CUDA(ctx, F.lightRec.reserve(std::max<size_t>(1, em.size()) * (80 + 32)));
   NOMAD_CUDA(ctx, F.lightCdf.reserve(std::max<size_t>(1, em.size()) * 4));
   NOMAD_CUDA(ctx, F.lightPdf.reserve((size_t)P * 4));
   NOMAD_CUDA(ctx, F.lightMeta.reserve(sizeof(LightMeta)));

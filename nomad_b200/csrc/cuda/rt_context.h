@@ -55,7 +55,7 @@ struct FrameState {
   DeviceBuf counters;                 // queue lengths, cursors, statistics
   DeviceBuf views;                    // view table
   DeviceBuf lightIdx, lightCdf, lightPdf, lightMeta;
-  DeviceBuf lightRec;                 // per CDF slot, 5 float4 (pt_lights.cuh)
+  DeviceBuf lightRec;                 // 5 float4 per CDF slot, then 2 for culling (pt_lights.cuh)
   bool lightsDirty = true;
   // ReSTIR DI: per-path reservoirs (initial, temporal, final of this and the previous frame),
   // surface records (this and the previous frame) and the previous frame's view table
@@ -63,6 +63,7 @@ struct FrameState {
   uint64_t restirPaths = 0;
   int restirCur = 0;
   bool restirValid = false;
+  bool restirSmemSet = false;  // k_restir_initial opted in to its shared memory
   nomad_restir_config restir{32, 1, 3, 30.0f, 20.0f, 0};
   // reference-mode ReSTIR: candidate and reuse visibility queues, per-path visibility masks,
   // the selected contribution after the candidates
