@@ -119,7 +119,7 @@ __device__ __forceinline__ void light_cull(const float4 *__restrict__ prims, uin
   if (s.type == 1) {
     q[0] = s.a;
     q[1] = s.b;
-    q[2] = s.c;
+    q[2] = q[3] = s.c;
     n = 3;
   } else {
     q[0] = s.a + s.b + s.c;
@@ -129,10 +129,14 @@ __device__ __forceinline__ void light_cull(const float4 *__restrict__ prims, uin
     n = 4;
   }
   V3 mid = q[0];
-  for (int i = 1; i < n; ++i) mid = mid + q[i];
+#pragma unroll
+  for (int i = 1; i < 4; ++i)
+    if (i < n) mid = mid + q[i];
   mid = mid * (n == 3 ? 1.0f / 3.0f : 0.25f);
   float least = INFINITY, radius = 0.0f, size = 0.0f;
-  for (int i = 0; i < n; ++i) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (i >= n) break;
     least = fminf(least, dot(s.nrm, q[i]));
     radius = fmaxf(radius, length(q[i] - mid));
     size = fmaxf(size, fabsf(q[i].x) + fabsf(q[i].y) + fabsf(q[i].z));

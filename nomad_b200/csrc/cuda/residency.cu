@@ -212,26 +212,27 @@ __device__ __forceinline__ unsigned long long block_exscan64(unsigned long long 
   return r;
 }
 
-// After the sort each key holds (object bytes / 4) in its high word and the object in its low
-// word. Object bytes are 32 per node + 196 per primitive, so always a multiple of 4, and
+// In score order each entry holds (object bytes / 4) in its high word, the object in its low one and
+// whether the object is visible in bit 31. Object bytes are 32 per node + 196 per primitive, so always a multiple of 4, and
 // "used + b <= budget" holds exactly when "used/4 + b/4 <= budget/4" (rounded down).
-__device__ __forceinline__ uint32_t key_obj(unsigned long long k) { return (uint32_t)(k & 0xffffffffu); }
+__device__ __forceinline__ uint32_t key_obj(unsigned long long k) { return (uint32_t)k & 0x7fffffffu; }
+__device__ __forceinline__ bool key_visible(unsigned long long k) { return ((uint32_t)k >> 31) != 0; }
 __device__ __forceinline__ unsigned long long key_b4(unsigned long long k) { return k >> 32; }
 
-// Greedy fill in sorted order from position `from` by one warp: candidates are taken while they
-// fit, skipping those that do not (the sequential rule), 32 positions at a time. Each round
+// Greedy fill by one warp over the m listed positions, which ascend in score order: candidates are taken
+// while they fit, skipping those that do not (the sequential rule), 32 positions at a time. Each round
 // first drops lanes that cannot fit on their own, then accepts the longest run of candidates
 // whose running total fits; the first candidate past that run is skipped.
-__device__ void warp_greedy(uint32_t from, uint32_t n, const unsigned long long *sk, unsigned long long budget4,
-                            bool unlimited, const uint8_t *cand, uint8_t *dsel, unsigned long long *used4) {
+__device__ void warp_greedy(uint32_t m, const uint16_t *list, const unsigned long long *sk,
+                            unsigned long long budget4, uint8_t *dsel, unsigned long long *used4) {
   const unsigned lane = threadIdx.x & 31u;
   unsigned long long u = *used4;
-  for (uint32_t base = from; base < n; base += 32) {
-    const uint32_t k = base + lane;
-    bool c = k < n && cand[k];
+  for (uint32_t base = 0; base < m; base += 32) {
+    bool c = base + lane < m;
+    const uint32_t k = c ? list[base + lane] : 0u;
     const unsigned long long b = c ? key_b4(sk[k]) : 0ull;
     for (;;) {
-      const unsigned long long rem = unlimited ? ~0ull : (u > budget4 ? 0ull : budget4 - u);
+      const unsigned long long rem = u > budget4 ? 0ull : budget4 - u;
       if (c && b > rem) c = false;
       if (__ballot_sync(0xffffffffu, c) == 0) break;
       unsigned long long p = c ? b : 0ull;  // inclusive prefix of candidate bytes
@@ -256,110 +257,156 @@ struct SelectShared {
   unsigned long long warpSums64[32];
   unsigned long long total64;
   unsigned long long used4;
-  unsigned long long add4;
   uint32_t warpSums[32];
   uint32_t total;
   uint32_t first;
+  uint32_t listed;
 };
 
-// One budget walk over the candidates (cand[k] = 1) in sorted order, with the whole block: a
-// block scan of candidate bytes finds the first candidate that no longer fits; every candidate
-// before it is taken at once, that one is skipped, and one warp finishes the walk after it
-// (where the remaining budget is below that candidate's size, so most objects drop at once).
+// One budget walk over the candidates (cand[k] = 1) in sorted order, with the whole block. A round
+// drops the candidates above the budget left (it only shrinks), scans the bytes of the others and
+// takes all before the first that no longer fits; the next round starts after that one. Each round's failing
+// candidate is smaller than the last one's, so 2,048 objects of mixed sizes need 3 to 6 rounds (about
+// 1.3 us each); should kWalkRounds not do, one warp finishes over the list of those that still fit.
+// The warp alone after one round takes the same time at 2,048 objects, but its time grows with them.
+constexpr int kWalkRounds = 12;
 __device__ void budget_walk(uint32_t n, uint32_t npow2, const unsigned long long *sk, unsigned long long budget4,
-                            bool unlimited, const uint8_t *cand, uint8_t *dsel, SelectShared &sh) {
+                            bool unlimited, const uint8_t *cand, uint8_t *dsel, uint16_t *list,
+                            SelectShared &sh) {
   const uint32_t per = (npow2 + blockDim.x - 1) / blockDim.x;
   const uint32_t k0 = threadIdx.x * per, k1 = min(k0 + per, n);
-  unsigned long long seg = 0;
-  for (uint32_t k = k0; k < k1; ++k)
-    if (cand[k]) seg += key_b4(sk[k]);
-  if (threadIdx.x == 0) sh.first = npow2;
-  const unsigned long long excl = block_exscan64(seg, sh.warpSums64, &sh.total64);  // syncs inside
-  const unsigned long long u0 = sh.used4;
-  const unsigned long long rem = unlimited ? ~0ull : (u0 > budget4 ? 0ull : budget4 - u0);
-  unsigned long long run = excl;
-  for (uint32_t k = k0; k < k1; ++k) {
-    if (!cand[k]) continue;
-    run += key_b4(sk[k]);
-    if (run > rem) {
-      atomicMin(&sh.first, k);
-      break;
+  uint32_t from = k0;  // this thread's first position that is still open
+  unsigned long long left;
+  auto open = [&](uint32_t k) { return cand[k] && key_b4(sk[k]) <= left; };
+  for (int round = 0;; ++round) {
+    const unsigned long long u0 = sh.used4;
+    left = unlimited ? ~0ull : (u0 > budget4 ? 0ull : budget4 - u0);
+    if (round == kWalkRounds) break;
+    unsigned long long seg = 0;
+    for (uint32_t k = from; k < k1; ++k)
+      if (open(k)) seg += key_b4(sk[k]);
+    if (threadIdx.x == 0) sh.first = npow2;
+    unsigned long long run = block_exscan64(seg, sh.warpSums64, &sh.total64);  // syncs inside
+    if (run + seg > left) {
+      for (uint32_t k = from; k < k1; ++k) {
+        if (!open(k)) continue;
+        if (run + key_b4(sk[k]) > left) {
+          atomicMin(&sh.first, k);
+          break;
+        }
+        run += key_b4(sk[k]);
+      }
     }
+    __syncthreads();
+    const uint32_t R = sh.first;
+    for (uint32_t k = from; k < k1 && k < R; ++k)
+      if (open(k)) dsel[k] = 1;
+    if (R >= npow2) {  // all of them fit
+      if (threadIdx.x == 0) sh.used4 = u0 + sh.total64;
+      __syncthreads();
+      return;
+    }
+    if (k0 <= R && R < k0 + per) sh.used4 = u0 + run;  // the segment holding R: run is the bytes before it
+    from = max(k0, R + 1);
+    __syncthreads();
   }
+  uint32_t fits = 0;
+  for (uint32_t k = from; k < k1; ++k) fits += open(k) ? 1u : 0u;
+  uint32_t at = block_exscan(fits, sh.warpSums, &sh.listed);
+  for (uint32_t k = from; k < k1; ++k)
+    if (open(k)) list[at++] = (uint16_t)k;
   __syncthreads();
-  const uint32_t R = sh.first;
-  unsigned long long before = excl;  // candidate bytes before R inside this segment
-  for (uint32_t k = k0; k < k1 && k < R; ++k)
-    if (cand[k]) {
-      dsel[k] = 1;
-      before += key_b4(sk[k]);
-    }
-  if (R < npow2 && k0 <= R && R < k0 + per) sh.add4 = before;  // the segment holding R
-  if (R >= npow2 && threadIdx.x == 0) sh.add4 = sh.total64;
-  __syncthreads();
-  if (threadIdx.x == 0) sh.used4 = u0 + sh.add4;
-  __syncthreads();
-  if (R + 1 < n && threadIdx.x < 32) warp_greedy(R + 1, n, sk, budget4, unlimited, cand, dsel, &sh.used4);
+  if (threadIdx.x < 32) warp_greedy(sh.listed, list, sk, budget4, dsel, &sh.used4);
   __syncthreads();
 }
 
-// Light CDF over the emissive primitives whose primitive is active and whose object is
-// resident, summed sequentially in primitive order (one thread; the flags are gathered by the
-// block first). Also writes the per-primitive light pdf used by ReSTIR. Called by one block.
+// Light CDF over the emissive primitives whose primitive is active and whose object is resident, summed
+// sequentially in primitive order (that order is the result's): the block gathers flags, weights
+// and slots, one thread only adds, from shared memory. With the whole loop on one thread each
+// light waited for its own global loads (64 lights: 8 of k_select's 59 us). Also writes the
+// per-primitive light pdf used by ReSTIR. Called by one block of 1,024 threads.
+constexpr uint32_t kLightChunk = 4096;
+struct alignas(16) LightShared {
+  float sum[kLightChunk];  // weights, then running totals
+  uint32_t warpSums[32];
+  uint32_t count, add;
+  float total;
+};
+
 __device__ void lights_rebuild(const uint4 *__restrict__ em, uint32_t ne, const uint8_t *__restrict__ primAct,
                                const uint8_t *objRes, uint32_t *__restrict__ idx, float *__restrict__ cdf,
-                               float *__restrict__ pdf, LightMeta *__restrict__ meta, uint8_t *on, float &total_s,
-                               uint32_t &count_s, const float4 *__restrict__ prims, const float4 *__restrict__ mats,
+                               float *__restrict__ pdf, LightMeta *__restrict__ meta, LightShared &sh,
+                               const float4 *__restrict__ prims, const float4 *__restrict__ mats,
                                float4 *__restrict__ rec) {
   if (threadIdx.x == 0) {
-    total_s = 0.0f;
-    count_s = 0;
+    sh.total = 0.0f;
+    sh.count = 0;
   }
   __syncthreads();
-  for (uint32_t base = 0; base < ne; base += 4096) {
-    uint32_t m = min(4096u, ne - base);
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-      uint4 e = em[base + i];
-      on[i] = primAct[e.x] && objRes[e.z];
+  constexpr uint32_t kPer = kLightChunk / 1024;
+  for (uint32_t base = 0; base < ne; base += kLightChunk) {
+    const uint32_t m = min(kLightChunk, ne - base), i0 = threadIdx.x * kPer;
+    uint32_t prim[kPer], on = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k) {
+      const uint32_t i = i0 + k;
+      float w = 0.0f;
+      if (i < m) {
+        const uint4 e = em[base + i];
+        prim[k] = e.x;
+        pdf[e.x] = 0.0f;
+        if (primAct[e.x] && objRes[e.z]) {
+          on |= 1u << k;
+          w = __uint_as_float(e.y);
+        }
+      }
+      sh.sum[i] = w;  // a primitive that is off adds 0, which leaves the total as it is
+    }
+    uint32_t c = block_exscan(__popc(on), sh.warpSums, &sh.add);  // syncs
+    if (threadIdx.x == 0) {
+      float total = sh.total;
+      for (uint32_t i = 0; i < (m + 3u) / 4u; ++i) {
+        float4 v = reinterpret_cast<float4 *>(sh.sum)[i];
+        v.x = total += v.x;
+        v.y = total += v.y;
+        v.z = total += v.z;
+        v.w = total += v.w;
+        reinterpret_cast<float4 *>(sh.sum)[i] = v;
+      }
+      sh.total = total;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float total = total_s;
-      uint32_t c = count_s;
-      for (uint32_t i = 0; i < m; ++i) {
-        uint4 e = em[base + i];
-        pdf[e.x] = 0.0f;
-        if (!on[i]) continue;
-        total += __uint_as_float(e.y);
-        idx[c] = e.x;
-        cdf[c] = total;
+    c += sh.count;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; ++k)
+      if (on >> k & 1u) {
+        idx[c] = prim[k];
+        cdf[c] = sh.sum[i0 + k];
         ++c;
       }
-      total_s = total;
-      count_s = c;
-    }
+    __syncthreads();
+    if (threadIdx.x == 0) sh.count += sh.add;
     __syncthreads();
   }
+  const uint32_t c = sh.count;
+  const float total = sh.total;
   if (threadIdx.x == 0) {
-    float total = total_s;
-    uint32_t c = count_s;
     meta->count = c;
     meta->total = total;
-    float prev = 0.0f;
-    for (uint32_t k = 0; k < c; ++k) {
-      float w = cdf[k] - prev;
-      prev = cdf[k];
-      if (w > 0.0f && total > 0.0f) pdf[idx[k]] = w / total;
-    }
   }
-  __syncthreads();
-  // light records of the new CDF (the weight of slot k is cdf[k] - cdf[k-1], as samplers read it)
-  const uint32_t c = count_s;
-  const float total = total_s;
-  for (uint32_t k = threadIdx.x; k < c; k += blockDim.x) {
-    const float prev = k > 0 ? cdf[k - 1] : 0.0f;
-    nomad_pt::light_record(prims, mats, idx[k], cdf[k] - prev, total, rec + 5ull * k);
-    nomad_pt::light_cull(prims, idx[k], rec + 5ull * ne + 2ull * k);  // behind the records
+  // Light pdf and records of the new CDF (the weight of slot k is cdf[k] - cdf[k-1], as samplers read
+  // it) by one half of the block, cull records (behind the records) by the other.
+  const uint32_t half = blockDim.x / 2;
+  if (threadIdx.x < half) {
+    for (uint32_t k = threadIdx.x; k < c; k += half) {
+      const float w = cdf[k] - (k > 0 ? cdf[k - 1] : 0.0f);
+      const uint32_t lp = idx[k];
+      if (w > 0.0f && total > 0.0f) pdf[lp] = w / total;
+      nomad_pt::light_record(prims, mats, lp, w, total, rec + 5ull * k);
+    }
+  } else {
+    for (uint32_t k = threadIdx.x - half; k < c; k += half)
+      nomad_pt::light_cull(prims, idx[k], rec + 5ull * ne + 2ull * k);
   }
 }
 
@@ -370,10 +417,8 @@ __global__ void __launch_bounds__(1024) k_lights_rebuild(const uint4 *__restrict
                                                          float *__restrict__ pdf, LightMeta *__restrict__ meta,
                                                          const float4 *__restrict__ prims,
                                                          const float4 *__restrict__ mats, float4 *__restrict__ rec) {
-  __shared__ uint8_t on[4096];
-  __shared__ float total_s;
-  __shared__ uint32_t count_s;
-  lights_rebuild(em, ne, primAct, objRes, idx, cdf, pdf, meta, on, total_s, count_s, prims, mats, rec);
+  __shared__ LightShared ls;
+  lights_rebuild(em, ne, primAct, objRes, idx, cdf, pdf, meta, ls, prims, mats, rec);
 }
 
 // Wide-layout instance slots that one step rewrites (4- and 8-wide).
@@ -396,58 +441,72 @@ struct LightArgs {
   float4 *rec;
 };
 
-// Single block of 1024 threads, the whole residency decision of one step: sort by score, select
+// Score order of the objects: each warp counts, for 32 objects, the keys below theirs in its share of
+// the tile, so an object's rank is the sum over the block's warps. Counting over the whole chip
+// takes n^2 / 32 warp steps, 6 us with its launch for 2,048 objects; the bitonic sort of one block that it
+// replaces was bound by shared-memory passes (66 of them: 15 us). Bound by latency: two dependent
+// loads, one tile and two barriers. With this, the rounds of budget_walk and the light sums, a step's
+// decision takes 33 us instead of 59 (2,048 objects, 64 lights).
+constexpr uint32_t kRankTile = 2048;
+__global__ void __launch_bounds__(1024) k_rank(uint32_t n, uint32_t policy, const float *__restrict__ keys,
+                                               const uint8_t *__restrict__ visible,
+                                               const unsigned long long *__restrict__ bytes, float resBonus,
+                                               const uint8_t *__restrict__ res,
+                                               unsigned long long *__restrict__ order) {
+  __shared__ unsigned long long tile[kRankTile];
+  __shared__ uint32_t part[32][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  auto key_of = [&](uint32_t i) {
+    float k = 1.0f;
+    if (policy != NOMAD_POLICY_ALWAYS) {
+      k = keys[i];
+      if (resBonus != 0.0f && res[i]) k = k + resBonus * fabsf(k);  // hysteresis for resident objects
+    }
+    return sort_key(k, i);
+  };
+  const uint32_t o = blockIdx.x * 32u + lane;
+  const unsigned long long mine = o < n ? key_of(o) : 0ull;
+  uint32_t below = 0;
+  for (uint32_t base = 0; base < n; base += kRankTile) {
+    const uint32_t m = min(kRankTile, n - base);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kRankTile; i += blockDim.x) tile[i] = i < m ? key_of(base + i) : ~0ull;
+    __syncthreads();
+    const unsigned long long *t = tile + warp * (kRankTile / 32);
+#pragma unroll 8
+    for (uint32_t i = 0; i < kRankTile / 32; ++i) below += t[i] < mine ? 1u : 0u;
+  }
+  part[warp][lane] = below;
+  __syncthreads();
+  if (warp == 0 && o < n) {
+    uint32_t rank = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) rank += part[w][lane];
+    order[rank] = ((unsigned long long)(bytes[o] >> 2) << 32) | (visible[o] ? 0x80000000u : 0u) | o;
+  }
+}
+
+// Single block of 1024 threads, the whole residency decision of one step: select in score order
 // under the budget (min_active, visibility reserve, fill), apply toggles in index order, patch the
 // instance links of the pair and wide layouts, and rebuild the light CDF over the new resident set.
 __global__ void __launch_bounds__(1024) k_select(uint32_t n, uint32_t npow2, uint32_t policy,
-                                                 const float *__restrict__ keys, const uint8_t *__restrict__ visible,
-                                                 const unsigned long long *__restrict__ bytes,
+                                                 const unsigned long long *__restrict__ order,
                                                  unsigned long long budget, uint32_t reserve, uint32_t minActive,
-                                                 uint32_t maxToggles, float resBonus, uint8_t *__restrict__ desired,
+                                                 uint32_t maxToggles, uint8_t *__restrict__ desired,
                                                  uint8_t *__restrict__ res, const long long *__restrict__ slot,
                                                  const int32_t *__restrict__ blasRef, int32_t *__restrict__ pnodeWords,
                                                  uint32_t *__restrict__ misc, WidePatch wp, LightArgs la) {
   extern __shared__ unsigned long long sk[];
   uint8_t *dsel = reinterpret_cast<uint8_t *>(sk + npow2);  // selected, by sorted position
   uint8_t *cand = dsel + npow2;                             // candidates of the current walk
+  uint16_t *list = reinterpret_cast<uint16_t *>(cand + npow2);  // positions left to its greedy part
   __shared__ SelectShared sh;
-  __shared__ uint8_t on[4096];
-  __shared__ float ltotal;
-  __shared__ uint32_t lcount;
-  for (uint32_t i = threadIdx.x; i < npow2; i += blockDim.x) {
-    float k = 1.0f;
-    if (i < n && policy != NOMAD_POLICY_ALWAYS) {
-      k = keys[i];
-      if (resBonus != 0.0f && res[i]) k = k + resBonus * fabsf(k);  // hysteresis for resident objects
-    }
-    sk[i] = i < n ? sort_key(k, i) : ~0ull;
-  }
+  __shared__ LightShared ls;
   if (threadIdx.x == 0) {
     sh.used4 = 0;
     misc[1] = 0;
   }
-  __syncthreads();
-  for (uint32_t k = 2; k <= npow2; k <<= 1) {
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < npow2; i += blockDim.x) {
-        uint32_t l = i ^ j;
-        if (l > i) {
-          unsigned long long a = sk[i], b = sk[l];
-          bool up = (i & k) == 0;
-          if ((a > b) == up) {
-            sk[i] = b;
-            sk[l] = a;
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // sorted keys -> (bytes / 4, object)
-  for (uint32_t k = threadIdx.x; k < npow2; k += blockDim.x) {
-    const uint32_t o = (uint32_t)(sk[k] & 0xffffffffu);
-    sk[k] = k < n ? ((unsigned long long)(bytes[o] >> 2) << 32) | o : 0ull;
-  }
+  for (uint32_t k = threadIdx.x; k < npow2; k += blockDim.x) sk[k] = k < n ? order[k] : 0ull;
   __syncthreads();
   const bool unlimited = budget == 0 || policy == NOMAD_POLICY_ALWAYS;
   const unsigned long long budget4 = budget >> 2;
@@ -463,22 +522,22 @@ __global__ void __launch_bounds__(1024) k_select(uint32_t n, uint32_t npow2, uin
   const uint32_t per = (npow2 + blockDim.x - 1) / blockDim.x;
   const uint32_t k0 = threadIdx.x * per;
   uint32_t nv = 0;
-  for (uint32_t k = k0; k < k0 + per && k < n; ++k) nv += visible[key_obj(sk[k])] ? 1u : 0u;
+  for (uint32_t k = k0; k < k0 + per && k < n; ++k) nv += key_visible(sk[k]) ? 1u : 0u;
   uint32_t before = block_exscan(nv, sh.warpSums, &sh.total);
   for (uint32_t k = k0; k < k0 + per && k < npow2; ++k) {
     bool c = false;
-    if (k < n && visible[key_obj(sk[k])]) {
+    if (k < n && key_visible(sk[k])) {
       c = before < reserve && !dsel[k];
       ++before;
     }
     cand[k] = c ? 1 : 0;
   }
   __syncthreads();
-  budget_walk(n, npow2, sk, budget4, unlimited, cand, dsel, sh);
+  budget_walk(n, npow2, sk, budget4, unlimited, cand, dsel, list, sh);
   // fill in score order
   for (uint32_t k = threadIdx.x; k < npow2; k += blockDim.x) cand[k] = (k < n && !dsel[k]) ? 1 : 0;
   __syncthreads();
-  budget_walk(n, npow2, sk, budget4, unlimited, cand, dsel, sh);
+  budget_walk(n, npow2, sk, budget4, unlimited, cand, dsel, list, sh);
   for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) desired[key_obj(sk[k])] = dsel[k];
   __syncthreads();
   // toggles in index order, the first max_toggles of them when bounded
@@ -492,20 +551,28 @@ __global__ void __launch_bounds__(1024) k_select(uint32_t n, uint32_t npow2, uin
     ++rank;
     if (!apply) continue;
     res[o] = want;
+    // every address and value first, so that their loads overlap
     const long long s = slot[o];
-    const int32_t ref = want ? blasRef[o] : kEmptyRef;
+    const int32_t ref = blasRef[o];
+    long long ws[2];
+    int32_t wref[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      ws[w] = wp.width[w] ? wp.slot[w][o] : -1;
+      wref[w] = wp.width[w] ? wp.ref[w][o] : kEmptyRef;
+    }
     if (s >= 0) {
-      pnodeWords[(s / 2) * 16 + ((s & 1) ? 7 : 3)] = ref;
+      pnodeWords[(s / 2) * 16 + ((s & 1) ? 7 : 3)] = want ? ref : kEmptyRef;
     } else if (s == -1) {
       misc[1] = 1;
       misc[2] = want;
     }
+#pragma unroll
     for (int w = 0; w < 2; ++w) {
-      if (!wp.width[w]) continue;
-      const long long ws = wp.slot[w][o];
-      if (ws < 0) continue;
-      wp.arena[wp.base[w] + (size_t)(ws / wp.width[w]) * wp.fpn[w] + 6 * wp.width[w] + (size_t)(ws % wp.width[w])] =
-          want ? wp.ref[w][o] : kEmptyRef;
+      if (ws[w] < 0) continue;
+      const int lg = __ffs(wp.width[w]) - 1;  // 4 or 8 wide
+      wp.arena[wp.base[w] + (size_t)(ws[w] >> lg) * wp.fpn[w] + 6 * wp.width[w] + (size_t)(ws[w] & (wp.width[w] - 1))] =
+          want ? wref[w] : kEmptyRef;
     }
   }
   if (threadIdx.x == 0) {
@@ -514,8 +581,7 @@ __global__ void __launch_bounds__(1024) k_select(uint32_t n, uint32_t npow2, uin
     misc[3] = 0;
   }
   __syncthreads();  // res[] complete for the light rebuild
-  lights_rebuild(la.em, la.ne, la.primAct, res, la.idx, la.cdf, la.pdf, la.meta, on, ltotal, lcount, la.prims, la.mats,
-                 la.rec);
+  lights_rebuild(la.em, la.ne, la.primAct, res, la.idx, la.cdf, la.pdf, la.meta, ls, la.prims, la.mats, la.rec);
 }
 
 float luminance_host(const float *c) { return c[0] * 0.2126f + c[1] * 0.7152f + c[2] * 0.0722f; }
@@ -556,6 +622,7 @@ nomad_status nomad_residency_init(nomad_ctx *ctx) {
   NOMAD_CUDA(ctx, R.visible.reserve(N));
   NOMAD_CUDA(ctx, R.features.reserve((size_t)N * NOMAD_FEATURES * 4));
   NOMAD_CUDA(ctx, R.keys.reserve((size_t)N * 4));
+  NOMAD_CUDA(ctx, R.order.reserve((size_t)N * 8));
   NOMAD_CUDA(ctx, R.desired.reserve(N));
   NOMAD_CUDA(ctx, R.misc.reserve(64));
   NOMAD_CUDA(ctx, cudaMemcpy(R.objSlot.p, L.objSlot.data(), (size_t)N * 8, cudaMemcpyHostToDevice));
@@ -2194,8 +2261,8 @@ extern "C" nomad_status nomad_residency_step(nomad_ctx *ctx, const nomad_residen
   }
   uint32_t npow2 = 1;
   while (npow2 < N) npow2 <<= 1;
-  size_t smem = (size_t)npow2 * 10;  // sort keys, selected and candidate flags
-  if (smem > 48 * 1024)
+  size_t smem = (size_t)npow2 * 12;  // entries, selected and candidate flags, greedy list
+  if (smem > 24 * 1024)  // with the 18 KB of static shared memory beyond the default limit
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   float motion = std::min(std::max(prm->camera_motion, 0.0f), 1.0f);
   uint32_t reserve = (uint32_t)std::min<double>(N, std::ceil(N * (prm->reserve_base + prm->reserve_motion * motion)));
@@ -2214,10 +2281,13 @@ extern "C" nomad_status nomad_residency_step(nomad_ctx *ctx, const nomad_residen
   LightArgs la{R.emissive.as<const uint4>(), R.emissiveCount, R.primAct.as<const uint8_t>(), F.lightIdx.as<uint32_t>(),
                F.lightCdf.as<float>(), F.lightPdf.as<float>(), F.lightMeta.as<LightMeta>(),
                ctx->prims.as<const float4>(), ctx->materials.as<const float4>(), F.lightRec.as<float4>()};
+  k_rank<<<(N + 31) / 32, 1024, 0, s>>>(N, prm->policy, R.keys.as<const float>(), R.visible.as<const uint8_t>(),
+                                        R.bytes.as<const unsigned long long>(), prm->resident_key_bonus,
+                                        R.objRes.as<const uint8_t>(), R.order.as<unsigned long long>());
+  NOMAD_CUDA(ctx, cudaGetLastError());
   // one kernel: selection, toggles, pair and wide layout patches, light CDF
-  k_select<<<1, 1024, smem, s>>>(N, npow2, prm->policy, R.keys.as<const float>(), R.visible.as<const uint8_t>(),
-                                 R.bytes.as<const unsigned long long>(), prm->budget_bytes, reserve, prm->min_active,
-                                 prm->max_toggles, prm->resident_key_bonus, R.desired.as<uint8_t>(),
+  k_select<<<1, 1024, smem, s>>>(N, npow2, prm->policy, R.order.as<const unsigned long long>(), prm->budget_bytes,
+                                 reserve, prm->min_active, prm->max_toggles, R.desired.as<uint8_t>(),
                                  R.objRes.as<uint8_t>(),
                                  R.objSlot.as<const long long>(), R.objBlasRef.as<const int32_t>(),
                                  static_cast<int32_t *>(ctx->arena.p), R.misc.as<uint32_t>(), wp, la);

@@ -144,6 +144,7 @@ struct nomad_ctx {
     DeviceBuf bounds, bytes, tris, emit;               // float4 (centre, radius), u64, u32, f32
     DeviceBuf score, hist, lastHit, prevDist, visible; // f32, u32[8], u32, f32, u8
     DeviceBuf features, keys, desired, misc;           // f32[24], f32, u8, misc words
+    DeviceBuf order;                                   // u64 per object, in score order (k_rank)
     DeviceBuf emissive;                                // {prim, weight bits, object} per emissive primitive
     uint32_t emissiveCount = 0;
     uint32_t frame = 0;
