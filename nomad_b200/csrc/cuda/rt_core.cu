@@ -608,7 +608,8 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
         chunk = (uint32_t)std::min<uint64_t>(128, (share + 31) & ~31ull);
       const uint64_t warps = chunk ? (m + chunk - 1) / chunk : std::min<uint64_t>((uint64_t)ctx->smCount * perSm * (kBlock / 32), (m + 31) / 32);
       const uint64_t blocks = (warps + kBlock / 32 - 1) / (kBlock / 32);
-      if (!chunk) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
+      // callers with a queue on the device clear its cursor there, with the queue's length
+      if (!chunk && !lenDev) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
       kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays + 2 * off, m, lenDev, chunk ? nullptr : cursor,
                                                 hits5 ? hits5 + 5 * off : nullptr, occ ? occ + off : nullptr, counts,
                                                 chunk);
