@@ -46,6 +46,13 @@ struct ViewDev {
   unsigned long long pathOffset, pixelOffset;
 };
 
+// Tile pixel and sample of a path; a frame has fewer than 2^32 of them.
+__device__ __forceinline__ void split_path(const ViewDev &v, unsigned long long pid, uint32_t &pixel, uint32_t &sample) {
+  const uint32_t local = (uint32_t)(pid - v.pathOffset);
+  pixel = local / v.spp;
+  sample = local - pixel * v.spp;
+}
+
 // The view pixel of the tile's pixel lp (row-major in the tile): the index that keys the path's
 // random numbers and places its camera ray, so a tile's paths are the full view's paths.
 __device__ __forceinline__ uint32_t tile_pixel(const ViewDev &v, uint32_t lp) {
@@ -53,13 +60,15 @@ __device__ __forceinline__ uint32_t tile_pixel(const ViewDev &v, uint32_t lp) {
   return (v.ty + lp / v.tw) * v.w + v.tx + lp % v.tw;
 }
 
-// Queue lengths 128 bytes apart: every warp of k_shade appends to the next-bounce and the shadow
+// Queue lengths 128 bytes apart: every block of k_shade appends to the next-bounce and the shadow
 // queue, and atomics to one cache line are serialised by one L2 slice.
 constexpr int kQ = 32;
-// Resident blocks per SM the shading kernel is compiled for: 4 (64 registers, about 110 bytes
-// spilled) hides more of its dependent loads than 2 uncapped (105 registers) or 3 (80) did; the
-// images are the same.
-constexpr int kShadeMinBlocks = 4;
+// The shading kernel's block, and the threads per SM that it is compiled for: 1,024 (64 registers, about
+// 90 bytes spilled) hides more of its dependent loads than 768 (80 registers, 4 % of a frame slower)
+// or 512 uncapped; the images are the same. A block appends to both queues at once: with 256 threads
+// an eighth of the atomics on one address and 2 % off a frame; 128 threads gain 1 % and 1,024
+// nothing (the whole SM then waits at one barrier).
+constexpr int kShadeBlock = 256, kShadeThreads = 1024;
 struct Counters {
   uint32_t qlen[4 * kQ];            // [kQ * k]: 0, 1 bounce queues; 2 shadow queue; 3 ReSTIR rays
   unsigned long long cursor[2];     // persistent-trace cursors (closest, any)
@@ -105,6 +114,40 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t *len, bool want) {
   return base + __popc(m & ((1u << lane) - 1u));
 }
 
+// Appends of a whole block to two queues: one atomic a queue and block instead of one a warp, both under
+// way at once. Every thread calls it the same number of times, `buf` alternating 0, 1.
+template <int BLOCK>
+struct BlockAppend {
+  uint32_t counts[2][BLOCK / 32], base[2][2];
+  uint32_t before[2][BLOCK / 32];
+};
+template <int BLOCK>
+__device__ __forceinline__ void block_append2(BlockAppend<BLOCK> &sh, uint32_t buf, uint32_t *lenA, uint32_t *lenB,
+                                              bool wantA, bool wantB, uint32_t &slotA, uint32_t &slotB) {
+  constexpr uint32_t kWarps = BLOCK / 32;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const uint32_t ma = __ballot_sync(0xffffffffu, wantA), mb = __ballot_sync(0xffffffffu, wantB);
+  if (lane == 0) sh.counts[buf][warp] = __popc(ma) | (uint32_t)__popc(mb) << 16;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t v = lane < kWarps ? sh.counts[buf][lane] : 0u;
+    uint32_t x = v;
+#pragma unroll
+    for (uint32_t d = 1; d < kWarps; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, x, kWarps - 1);
+    if (lane < kWarps) sh.before[buf][lane] = x - v;
+    if (lane == 0 && (total & 0xffffu)) sh.base[buf][0] = atomicAdd(lenA, total & 0xffffu);
+    if (lane == 1 && (total >> 16)) sh.base[buf][1] = atomicAdd(lenB, total >> 16);
+  }
+  __syncthreads();
+  const uint32_t b = sh.before[buf][warp];
+  slotA = sh.base[buf][0] + (b & 0xffffu) + __popc(ma & lt);
+  slotB = sh.base[buf][1] + (b >> 16) + __popc(mb & lt);
+}
+
 __global__ void __launch_bounds__(kPtBlock) k_raygen(const ViewDev *__restrict__ views, uint32_t nviews,
                                                       unsigned long long P, float4 *__restrict__ rays,
                                                       uint32_t *__restrict__ ids, float4 *__restrict__ thr,
@@ -112,8 +155,9 @@ __global__ void __launch_bounds__(kPtBlock) k_raygen(const ViewDev *__restrict__
   unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long pid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; pid < P; pid += stride) {
     const ViewDev &v = find_view(views, nviews, pid);
-    unsigned long long local = pid - v.pathOffset;
-    uint32_t pixel = tile_pixel(v, (uint32_t)(local / v.spp)), sample = (uint32_t)(local % v.spp);
+    uint32_t pixel, sample;
+    split_path(v, pid, pixel, sample);
+    pixel = tile_pixel(v, pixel);
     uint32_t px = pixel % v.w, py = pixel / v.w;
     U4 r = philox(U4{pixel, sample, 255u * 4u, v.index}, v.k0, v.k1);
     float ux = ((float)px + 0.5f) / (float)v.w;
@@ -295,37 +339,35 @@ __device__ __forceinline__ V3 scatter(V3 inDir, V3 normal, bool frontFace, const
     outDir = normal;
     return v3(0.0f, 0.0f, 0.0f);
   }
-  float xi = xiLobe * total;
-  if (xi < dw) {
-    // sampleCosineHemisphere (Scatter.h:54-71)
-    float r = sqrtf(fmax_ref(0.0f, u1));
-    float s, c;
-    sincos_turns(u2, s, c);
-    float x = r * c, y = r * s, z = sqrtf(fmax_ref(0.0f, 1.0f - u1));
-    V3 t, b;
-    onb(normal, t, b);
-    outDir = normalize(t * x + b * y + normal * z);
-    float prob = fmax_ref(dw / total, 1e-4f);
-    return m.diffuse * m.opacity / prob;
-  }
-  xi = xi - dw;
-  if (xi < sw) {
-    V3 refl = reflect(inDir, normal);
-    float exponent = fmax_ref(m.shininess, 1.0f);
-    if (m.roughness > 0.0f) {
-      float smooth = clamp01(1.0f - m.roughness);
-      float re = fmax_ref(1.0f, smooth * smooth * 256.0f);
-      exponent = fmax_ref(exponent, re);
+  const float xi = xiLobe * total;
+  const bool diffuse = xi < dw;
+  if (diffuse || xi - dw < sw) {
+    // The cosine hemisphere (sampleCosineHemisphere, Scatter.h:54-71) and the specular lobe around the
+    // mirror direction share all but the polar angle, so a warp with paths in both runs the
+    // sine, the basis and the two normalisations once.
+    const V3 axis = diffuse ? normal : reflect(inDir, normal);
+    float z, r2;
+    if (diffuse) {
+      r2 = u1;
+      z = sqrtf(fmax_ref(0.0f, 1.0f - u1));
+    } else {
+      float exponent = fmax_ref(m.shininess, 1.0f);
+      if (m.roughness > 0.0f) {
+        float smooth = clamp01(1.0f - m.roughness);
+        float re = fmax_ref(1.0f, smooth * smooth * 256.0f);
+        exponent = fmax_ref(exponent, re);
+      }
+      z = pow_pos(u1, 1.0f / (exponent + 1.0f));
+      r2 = 1.0f - z * z;
     }
-    float cosT = pow_pos(u1, 1.0f / (exponent + 1.0f));
-    float sinT = sqrtf(fmax_ref(0.0f, 1.0f - cosT * cosT));
+    const float r = sqrtf(fmax_ref(0.0f, r2));
     float s, c;
     sincos_turns(u2, s, c);
     V3 t, b;
-    onb(refl, t, b);
-    outDir = normalize(t * (sinT * c) + b * (sinT * s) + refl * cosT);
-    float prob = fmax_ref(sw / total, 1e-4f);
-    return m.specular / prob;
+    onb(axis, t, b);
+    outDir = normalize(t * (r * c) + b * (r * s) + axis * z);
+    const float prob = fmax_ref((diffuse ? dw : sw) / total, 1e-4f);
+    return (diffuse ? m.diffuse * m.opacity : m.specular) / prob;
   }
   float prob = fmax_ref(tw / total, 1e-4f);
   float eta = fmax_ref(m.ior, 1e-3f);
@@ -416,7 +458,10 @@ struct LightSearch {
   }
 };
 
-__global__ void __launch_bounds__(kPtBlock, kShadeMinBlocks) k_shade(
+// Bound by instruction issue and by gathers (54 % of the issue slots, half of the DRAM rate): the
+// lobes share their code (scatter), queues are appended by the block, and 64-bit divisions are gone.
+// 8.3M paths of a city frame with three bounces: 1.36 -> 1.02 ms of its three launches.
+__global__ void __launch_bounds__(kShadeBlock, kShadeThreads / kShadeBlock) k_shade(
     uint32_t depth, const ViewDev *__restrict__ views, uint32_t nviews, const float4 *__restrict__ qRays,
     const uint32_t *__restrict__ qIds, const int32_t *__restrict__ hits, float4 *__restrict__ nRays,
     uint32_t *__restrict__ nIds, float4 *__restrict__ sRays, uint32_t *__restrict__ sIds,
@@ -433,6 +478,7 @@ __global__ void __launch_bounds__(kPtBlock, kShadeMinBlocks) k_shade(
   // this thread's segments, escapes and hits, added to the frame's counters once at the end (one
   // atomic per warp and launch instead of three per warp and iteration on one cache line)
   uint32_t nSeg = 0, nEsc = 0, nHit = 0;
+  __shared__ BlockAppend<kShadeBlock> append;
   for (uint32_t it = 0; it < iters; ++it) {
     uint32_t i = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
     bool live = i < n;
@@ -461,8 +507,9 @@ __global__ void __launch_bounds__(kPtBlock, kShadeMinBlocks) k_shade(
       } else {
         hit = true;
         inst = h[0];
-        unsigned long long local = pid - v.pathOffset;
-        uint32_t pixel = tile_pixel(v, (uint32_t)(local / v.spp)), sample = (uint32_t)(local % v.spp);
+        uint32_t pixel, sample;
+        split_path(v, pid, pixel, sample);
+        pixel = tile_pixel(v, pixel);
         U4 b0 = philox(U4{pixel, sample, depth * 4u + 0u, v.index}, v.k0, v.k1);
         U4 b1 = philox(U4{pixel, sample, depth * 4u + 1u, v.index}, v.k0, v.k1);
         V3 p = v3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
@@ -471,8 +518,8 @@ __global__ void __launch_bounds__(kPtBlock, kShadeMinBlocks) k_shade(
         bool front = dot(nrm, d) < 0.0f;
         if (!front) nrm = -nrm;
         Material m = decode_material(matTable, (int32_t)(__float_as_uint(rec.w) & kShadeMatMask), v.lod);
-        float4 R = rad[pid];
         if (m.power * luminance(m.emission) > 0.0f) {
+          float4 R = rad[pid];
           R.x = R.x + tp.x * m.emission.x * m.power;
           R.y = R.y + tp.y * m.emission.y * m.power;
           R.z = R.z + tp.z * m.emission.z * m.power;
@@ -560,14 +607,14 @@ __global__ void __launch_bounds__(kPtBlock, kShadeMinBlocks) k_shade(
         if (hit && (threadIdx.x & 31) == __ffs(pp) - 1) atomicAdd(primHits + hitPrim, (uint32_t)__popc(pp));
       }
     }
-    uint32_t ss = warp_append(shadowLen, wantShadow);
+    uint32_t ss, ns;
+    block_append2<kShadeBlock>(append, it & 1u, shadowLen, nextLen, wantShadow, wantNext, ss, ns);
     if (wantShadow) {
       sRays[2 * ss] = sA;
       sRays[2 * ss + 1] = sB;
       sIds[ss] = pid;
       sContrib[ss] = sC;
     }
-    uint32_t ns = warp_append(nextLen, wantNext);
     if (wantNext) {
       nRays[2 * ns] = nA;
       nRays[2 * ns + 1] = nB;
@@ -910,7 +957,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
         rs = restir_launch(ctx, nviews, P, L, C, plan);
         if (rs != NOMAD_OK) return rs;
       }
-      k_shade<<<gridPT, kPtBlock, 0, s>>>(depth, V, nviews, F.qRays[cur].as<const float4>(),
+      k_shade<<<ctx->smCount * (kShadeThreads / kShadeBlock), kShadeBlock, 0, s>>>(depth, V, nviews, F.qRays[cur].as<const float4>(),
                                          F.qIds[cur].as<const uint32_t>(), F.hits.as<const int32_t>(),
                                          F.qRays[cur ^ 1].as<float4>(), F.qIds[cur ^ 1].as<uint32_t>(),
                                          F.sRays.as<float4>(), F.sIds.as<uint32_t>(), F.sContrib.as<float4>(),
@@ -1226,9 +1273,7 @@ __global__ void __launch_bounds__(kRiBlock, 1) k_restir_initial(
         }
       }
       sOut[pid] = s;
-      const unsigned long long local = pid - v.pathOffset;
-      pixel = (uint32_t)(local / v.spp);
-      sample = (uint32_t)(local % v.spp);
+      split_path(v, pid, pixel, sample);
       view = v.index;
       k0 = v.k0;
       k1 = v.k1;
@@ -1355,8 +1400,8 @@ __global__ void __launch_bounds__(kPtBlock) k_restir_temporal(
           float u = dot(rel, U) / dot(U, U), w = dot(rel, Vv) / dot(Vv, Vv);
           if (u >= 0.0f && u < 1.0f && w >= 0.0f && w < 1.0f) {
             uint32_t px = min((uint32_t)(u * (float)pv.w), pv.w - 1), py = min((uint32_t)(w * (float)pv.h), pv.h - 1);
-            unsigned long long local = pid - v.pathOffset;
-            uint32_t pixel = (uint32_t)(local / v.spp), sample = (uint32_t)(local % v.spp);
+            uint32_t pixel, sample;
+            split_path(v, pid, pixel, sample);
             unsigned long long ppid = pv.pathOffset + ((unsigned long long)py * pv.w + px) * pv.spp + sample;
             if (restir_gate(s, sPrev[ppid])) {
               const BsdfView b = bsdf_view(prim_material(mats, __float_as_int(s.n.w), v.lod), ld3(s.n), ld3(s.v));
@@ -1381,8 +1426,8 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_spatial(
     const Surf s = sCur[pid];
     if (s.v.w > 0.0f && cfg.spatial > 0) {
       const ViewDev &v = find_view(views, nviews, pid);
-      unsigned long long local = pid - v.pathOffset;
-      uint32_t pixel = (uint32_t)(local / v.spp), sample = (uint32_t)(local % v.spp);
+      uint32_t pixel, sample;
+      split_path(v, pid, pixel, sample);
       int px = (int)(pixel % v.w), py = (int)(pixel / v.w);
       const BsdfView b = bsdf_view(prim_material(mats, __float_as_int(s.n.w), v.lod), ld3(s.n), ld3(s.v));
       for (uint32_t k = 0; k < cfg.spatial; ++k) {
@@ -1633,9 +1678,7 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
           s.v = make_float4(vd.x, vd.y, vd.z, 1.0f);
         }
       }
-      unsigned long long local = pid - v.pathOffset;
-      pixel = (uint32_t)(local / v.spp);
-      sample = (uint32_t)(local % v.spp);
+      split_path(v, pid, pixel, sample);
       sOut[pid] = s;
       for (uint32_t w = 0; w < ra.words; ++w) mask[pid * ra.words + w] = 0u;
     }
@@ -1698,9 +1741,7 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_reuse(
       s = sCur[pid];
       const ViewDev &v = find_view(views, nviews, pid);
       vp = &v;
-      unsigned long long local = pid - v.pathOffset;
-      pixel = (uint32_t)(local / v.spp);
-      sample = (uint32_t)(local % v.spp);
+      split_path(v, pid, pixel, sample);
       Resv r = resv_empty();
       V3 contrib = v3(0.0f, 0.0f, 0.0f);
       if (s.v.w > 0.0f) {
@@ -1759,8 +1800,8 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_final(
       Resv r = rMid[pid];
       if (s.v.w > 0.0f) {
         const ViewDev &v = find_view(views, nviews, pid);
-        const unsigned long long local = pid - v.pathOffset;
-        const uint32_t pixel = (uint32_t)(local / v.spp), sample = (uint32_t)(local % v.spp);
+        uint32_t pixel, sample;
+        split_path(v, pid, pixel, sample);
         const BsdfView b = bsdf_view(prim_material(mats, __float_as_int(s.n.w), v.lod), ld3(s.n), ld3(s.v));
         const float4 mc = midContrib[pid];
         V3 contrib = v3(mc.x, mc.y, mc.z);
