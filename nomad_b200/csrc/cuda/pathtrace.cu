@@ -1642,13 +1642,38 @@ __device__ __forceinline__ bool ref_reuse_candidate(uint32_t k, const ViewDev &v
   return ref_stored_candidate(s, b, mats, ra, q, c);
 }
 
+// Rays of a warp on their way to the queue, written 32 at a time: one atomic on the queue's length for 32
+// rays and whole lines, where an append for each of a path's 32 candidates did 520,000 atomics on
+// one address (961x541: 297 us).
+struct RefRing {
+  float4 a[64], b[64];
+  uint32_t id[64];
+};
+
 __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
     const ViewDev *__restrict__ views, uint32_t nviews, unsigned long long P, RestirDev cfg,
     const float4 *__restrict__ rays, const int32_t *__restrict__ hits,
     const ShadeTables mats, Lights L, Surf *__restrict__ sOut, uint32_t *__restrict__ mask, RefArgs ra,
     float4 *__restrict__ qRays, uint32_t *__restrict__ qIds, Counters *cnt, uint32_t cdfCap) {
   extern __shared__ float4 lsShared[];
+  __shared__ RefRing rings[kPtBlock / 32];
   const LightSearch find(L, cdfCap, lsShared);
+  RefRing &ring = rings[threadIdx.x / 32];
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  uint32_t head = 0, done = 0;  // rays put into and written out of the warp's ring
+  auto write_out = [&](uint32_t count) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&cnt->qlen[kQ * (3)], count);
+    base = __shfl_sync(0xffffffffu, base, 0) + lane;  // the ring's entries are visible after this
+    if (lane < count) {
+      const uint32_t e = (done + lane) & 63u;
+      qRays[2ull * base] = ring.a[e];
+      qRays[2ull * base + 1] = ring.b[e];
+      qIds[base] = ring.id[e];
+    }
+    done += count;
+    __syncwarp();
+  };
   const uint32_t lightCount = find.count;
   const float lightTotal = find.total;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -1689,16 +1714,21 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
         const U4 u = philox(U4{pixel, sample, 0x10000u + c, vp->index}, vp->k0, vp->k1);
         want = ref_new_candidate(s, nullptr, L, find, u, cd);
       }
-      const uint32_t slot = warp_append(&cnt->qlen[kQ * (3)], want);
+      const uint32_t m = __ballot_sync(0xffffffffu, want);
       if (want) {
+        const uint32_t e = (head + __popc(m & lt)) & 63u;
         float4 A, B;
         ref_ray(s, cd, A, B);
-        qRays[2ull * slot] = A;
-        qRays[2ull * slot + 1] = B;
-        qIds[slot] = (uint32_t)(pid * cfg.candidates + c);
+        ring.a[e] = A;
+        ring.b[e] = B;
+        ring.id[e] = (uint32_t)(pid * cfg.candidates + c);
       }
+      head += __popc(m);
+      __syncwarp();
+      if (head - done >= 32) write_out(32);
     }
   }
+  if (head > done) write_out(head - done);
 }
 
 // Unoccluded entries of the visibility queue set their bit in the path's mask.
@@ -1960,6 +1990,13 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
   const int grid = ctx->smCount * 8;
   Surf *sCur = F.surf[cur].as<Surf>();
   const uint32_t cdfCap = std::min<uint32_t>(ctx->res.emissiveCount, kLsMost);  // lights staged in shared memory
+  if (!F.restirSmemSet) {
+    NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_restir_initial, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kRiFixed + ls_bytes(kLsMost))));
+    NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_restir_ref_cand, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)ls_bytes(kLsMost)));  // beside 18 KB of rings
+    F.restirSmemSet = true;
+  }
   if (cf.reference_mode) {
     const RefArgs ra{F.lightPdf.as<const float>(), ctx->primCount, (cf.candidates + 31) / 32};
     const ViewDev *PV = F.prevViews.as<const ViewDev>();
@@ -1995,11 +2032,6 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
     NOMAD_CUDA(ctx, cudaGetLastError());
     NOMAD_CUDA(ctx, cudaMemcpyAsync(F.prevViews.p, F.views.p, nviews * sizeof(ViewDev), cudaMemcpyDeviceToDevice, s));
     return NOMAD_OK;
-  }
-  if (!F.restirSmemSet) {
-    NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_restir_initial, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kRiFixed + ls_bytes(kLsMost))));
-    F.restirSmemSet = true;
   }
   k_restir_initial<<<ctx->smCount, kRiBlock, kRiFixed + ls_bytes(cdfCap), s>>>(
       V, nviews, P, cfg, F.qRays[0].as<const float4>(), F.hits.as<const int32_t>(),
