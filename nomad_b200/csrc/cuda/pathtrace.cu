@@ -460,7 +460,7 @@ struct LightSearch {
 
 // Bound by instruction issue and by gathers (54 % of the issue slots, half of the DRAM rate): the
 // lobes share their code (scatter), queues are appended by the block, and 64-bit divisions are gone.
-// 8.3M paths of a city frame with three bounces: 1.36 -> 1.02 ms of its three launches.
+// 8.3M paths of a city frame with three bounces: 1.36 -> 1.19 ms of its three launches.
 __global__ void __launch_bounds__(kShadeBlock, kShadeThreads / kShadeBlock) k_shade(
     uint32_t depth, const ViewDev *__restrict__ views, uint32_t nviews, const float4 *__restrict__ qRays,
     const uint32_t *__restrict__ qIds, const int32_t *__restrict__ hits, float4 *__restrict__ nRays,
@@ -1776,15 +1776,19 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_reuse(
       V3 contrib = v3(0.0f, 0.0f, 0.0f);
       if (s.v.w > 0.0f) {
         b = bsdf_view(prim_material(mats, __float_as_int(s.n.w), v.lod), ld3(s.n), ld3(s.v));
-        for (uint32_t c = 0; c < cfg.candidates; ++c) {
-          if (!((candMask[pid * ra.words + c / 32] >> (c % 32)) & 1u)) continue;
-          const U4 u = philox(U4{pixel, sample, 0x10000u + c, v.index}, v.k0, v.k1);
-          RefCand cd;
-          if (!ref_new_candidate(s, &b, L, find, u, cd)) continue;
-          const V3 cc = cd.radG / cd.pdf;
-          const float target = fmax_ref(luminance(cd.radG), 0.0f);
-          const float w = cd.pdf > 0.0f ? target / cd.pdf : 0.0f;
-          ref_update(r, contrib, cd, cc, w, 1.0f, u01(u.w));
+        // each lane walks its own visible candidates, so a warp takes as many steps as its path with the
+        // most of them, not one for every candidate that any of its paths sees
+        for (uint32_t w0 = 0; w0 < ra.words; ++w0) {
+          for (uint32_t left = candMask[pid * ra.words + w0]; left; left &= left - 1) {
+            const uint32_t c = w0 * 32 + __ffs(left) - 1;
+            const U4 u = philox(U4{pixel, sample, 0x10000u + c, v.index}, v.k0, v.k1);
+            RefCand cd;
+            if (!ref_new_candidate(s, &b, L, find, u, cd)) continue;
+            const V3 cc = cd.radG / cd.pdf;
+            const float target = fmax_ref(luminance(cd.radG), 0.0f);
+            const float w = cd.pdf > 0.0f ? target / cd.pdf : 0.0f;
+            ref_update(r, contrib, cd, cc, w, 1.0f, u01(u.w));
+          }
         }
       }
       rMid[pid] = r;
