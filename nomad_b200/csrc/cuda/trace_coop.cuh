@@ -14,7 +14,11 @@
 // spends most of its issue slots on leaves: lanes reach them at different steps, and a loop over
 // six records runs at 4 to 9 of 32 lanes. Measured on the 2.48M-triangle city, 4-wide nodes, the
 // per-lane persistent walk before and this one: 8.29M primary rays 1.19 -> 1.06 ms, 4.98M diffuse
-// bounces 2.18 -> 1.46 ms, 4.98M shadow any-hits 1.85 -> 1.24 ms.
+// bounces 2.18 -> 1.46 ms, 4.98M shadow any-hits 1.85 -> 1.21 ms.
+//
+// Any-hit walks take the nearest child first too (in slot order the shadows took 1.72 ms, the longest
+// overlap first 1.80, from the far end 2.25), but leave the other children unsorted and stack their refs
+// alone, as no distance is compared again: 1.24 -> 1.21 ms.
 //
 // The constants, each the fastest of those tried on the same rays:
 //   kCoopLeaves 8   leaf tests wait for eight leaves: 1.46 ms for the bounces; 4: 1.52, 12: 1.50.
@@ -48,6 +52,16 @@ struct CoopShared {
   uint32_t next[kCoopBlock / 32], left[kCoopBlock / 32];  // a warp's share of the batch not handed out yet
   int2 leaf[kCoopBlock];  // pending leaves of a warp: first record, lane of the ray
   int win[kCoopBlock];    // per ray: the lane whose hit is taken in this round
+};
+
+// What waits on a lane's stack: a ref and, for closest hits, the bits of its entry distance.
+template <bool ANY>
+struct alignas(ANY ? 4 : 8) StackEntry {
+  int32_t ref, t;
+};
+template <>
+struct StackEntry<true> {
+  int32_t ref;
 };
 
 // A ray as the node tests use it: origin, reciprocal direction and the rows of a wide node that hold
@@ -135,7 +149,7 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
   // Where boxes are cut off: tmax for any-hit, the closest hit's distance with the pruning margin
   // otherwise; kept finite, so that INFINITY marks a missed box.
   float bound = 0.0f;
-  int2 stk[STACK];  // (ref, bits of its entry distance)
+  StackEntry<ANY> stk[STACK];
   int sp = 0;
   int32_t ref = kEmptyRef;
   uint32_t ray = kNoRay;  // the lane's ray, until its result is stored
@@ -149,20 +163,28 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
   if (!cursor && sh.left[wb >> 5] == 0) return;
   for (;;) {
     while (ref == kEmptyRef && sp > 0) {  // the newest entry that still starts before the bound
-      const int2 e = stk[--sp];
-      ref = !ANY && __int_as_float(e.y) > bound ? kEmptyRef : e.x;
+      const StackEntry<ANY> e = stk[--sp];
+      ref = e.ref;
+      if constexpr (!ANY) ref = __int_as_float(e.t) > bound ? kEmptyRef : ref;
     }
     if (ref >= 0) {
       float t[W];
       int32_t c[W];
       coop_children<W>(S, WS, r, ref, bound, t, c);
-      sort_children<W>(t, c);
+      if constexpr (ANY && W == 4) {
+        cswap(t[0], c[0], t[1], c[1]);
+        cswap(t[2], c[2], t[3], c[3]);
+        cswap(t[0], c[0], t[2], c[2]);
+      } else {
+        sort_children<W>(t, c);
+      }
       // The upload sized the stack for W - 1 entries per level; the guard reports, not overruns.
       if (sp + W - 1 <= STACK) {
 #pragma unroll
         for (int k = W - 1; k >= 1; --k) {
           if (t[k] < INFINITY) {
-            stk[sp] = make_int2(c[k], __float_as_int(t[k]));
+            stk[sp].ref = c[k];
+            if constexpr (!ANY) stk[sp].t = __float_as_int(t[k]);
             ++sp;
           }
         }
@@ -326,10 +348,12 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
       }
       __syncwarp();
     }
-    if (!ANY && mine) {
-      bound = fminf(sh.o[tid].w * kPruneScale, FLT_MAX);
-      // entries that now start beyond the bound
-      while (sp > 0 && __int_as_float(stk[sp - 1].y) > bound) --sp;
+    if constexpr (!ANY) {
+      if (mine) {
+        bound = fminf(sh.o[tid].w * kPruneScale, FLT_MAX);
+        // entries that now start beyond the bound
+        while (sp > 0 && __int_as_float(stk[sp - 1].t) > bound) --sp;
+      }
     }
   }
 }
