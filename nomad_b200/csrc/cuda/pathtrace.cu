@@ -70,7 +70,8 @@ constexpr int kQ = 32;
 // nothing (the whole SM then waits at one barrier).
 constexpr int kShadeBlock = 256, kShadeThreads = 1024;
 struct Counters {
-  uint32_t qlen[4 * kQ];            // [kQ * k]: 0, 1 bounce queues; 2 shadow queue; 3 ReSTIR rays
+  uint32_t qlen[5 * kQ];            // [kQ * k]: 0, 1 bounce queues; 2, 4 shadow queue of even and odd
+                                    // depths; 3 ReSTIR rays
   unsigned long long cursor[2];     // persistent-trace cursors (closest, any)
   unsigned long long stats[4];      // segments, escapes, shadow rays, hits
   unsigned long long riNext;        // the next path of k_restir_initial
@@ -175,7 +176,12 @@ __global__ void __launch_bounds__(kPtBlock) k_raygen(const ViewDev *__restrict__
     thr[pid] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     rad[pid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cnt->qlen[kQ * (0)] = (uint32_t)P;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    cnt->qlen[kQ * 0] = (uint32_t)P;
+    cnt->qlen[kQ * 1] = cnt->qlen[kQ * 2] = cnt->qlen[kQ * 4] = 0;
+    cnt->cursor[0] = cnt->cursor[1] = 0;
+    cnt->riNext = 0;
+  }
 }
 
 struct Material {
@@ -466,13 +472,13 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeThreads / kShadeBlock) k_sh
     const uint32_t *__restrict__ qIds, const int32_t *__restrict__ hits, float4 *__restrict__ nRays,
     uint32_t *__restrict__ nIds, float4 *__restrict__ sRays, uint32_t *__restrict__ sIds,
     float4 *__restrict__ sContrib, float4 *__restrict__ thr, float4 *__restrict__ rad,
-    const float4 *__restrict__ shadeRec, const float4 *__restrict__ matTable, Lights L, Counters *cnt, int cur,
+    const float4 *__restrict__ shadeRec, const float4 *__restrict__ matTable, Lights L, Counters *cnt, int cur, int shadow,
     uint32_t *__restrict__ objHits, int restirDepth0, uint32_t *__restrict__ primHits) {
   const uint32_t n = cnt->qlen[kQ * (cur)];
   const uint32_t lightCount = L.meta->count;
   const float lightTotal = L.meta->total;
   uint32_t *nextLen = &cnt->qlen[kQ * (cur ^ 1)];
-  uint32_t *shadowLen = &cnt->qlen[kQ * (2)];
+  uint32_t *shadowLen = &cnt->qlen[kQ * shadow];
   uint32_t stride = gridDim.x * blockDim.x;
   uint32_t iters = (n + stride - 1) / stride;
   // this thread's segments, escapes and hits, added to the frame's counters once at the end (one
@@ -626,27 +632,25 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeThreads / kShadeBlock) k_sh
   warp_sum64(&cnt->stats[3], nHit);
 }
 
+// Adds the unoccluded lights' radiance. Also clears what the next bounce appends to and counts with: this
+// bounce's ray queue, the other shadow queue length and the trace cursors, all of which no
+// launch reads any more (a kernel of its own for that cost 2 us of each bounce).
 __global__ void __launch_bounds__(kPtBlock) k_resolve(const uint32_t *__restrict__ sIds,
                                                        const float4 *__restrict__ sContrib,
                                                        const uint8_t *__restrict__ occ, float4 *__restrict__ rad,
-                                                       Counters *cnt) {
-  uint32_t n = cnt->qlen[kQ * (2)];
+                                                       Counters *cnt, int cur, int shadow) {
+  uint32_t n = cnt->qlen[kQ * shadow];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (occ[i]) continue;
     uint32_t pid = sIds[i];
     float4 c = sContrib[i], R = rad[pid];
     rad[pid] = make_float4(R.x + c.x, R.y + c.y, R.z + c.z, R.w);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cnt->stats[2] += n;
-}
-
-// Clears the next-bounce and shadow queue lengths and the trace cursors before a bounce.
-__global__ void k_bounce_reset(Counters *cnt, int cur) {
-  cnt->qlen[kQ * (cur ^ 1)] = 0;
-  cnt->qlen[kQ * (2)] = 0;
-  cnt->cursor[0] = 0;
-  cnt->cursor[1] = 0;
-  cnt->riNext = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    cnt->stats[2] += n;
+    cnt->qlen[kQ * cur] = cnt->qlen[kQ * (6 - shadow)] = 0;
+    cnt->cursor[0] = cnt->cursor[1] = 0;
+  }
 }
 
 __global__ void __launch_bounds__(kPtBlock) k_finalize(const ViewDev *__restrict__ views, uint32_t nviews,
@@ -944,7 +948,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
     NOMAD_CUDA(ctx, cudaGetLastError());
     int cur = 0;
     for (uint32_t depth = 0; depth < maxDepth; ++depth) {
-      k_bounce_reset<<<1, 1, 0, s>>>(C, cur);
+      const int shadow = depth & 1 ? 4 : 2;
       nomad_status rs = nomad_trace_queue(ctx, false, F.qRays[cur].as<const float4>(), P, &C->qlen[kQ * (cur)],
                                             &C->cursor[0], F.hits.as<int32_t>(), nullptr, nullptr, s);
       if (rs != NOMAD_OK) return rs;
@@ -962,13 +966,13 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
                                          F.qRays[cur ^ 1].as<float4>(), F.qIds[cur ^ 1].as<uint32_t>(),
                                          F.sRays.as<float4>(), F.sIds.as<uint32_t>(), F.sContrib.as<float4>(),
                                          F.thr.as<float4>(), F.rad.as<float4>(), ctx->shadeRec.as<const float4>(),
-                                         ctx->matTable.as<const float4>(), L, C, cur, objHits, plan.on ? 1 : 0,
+                                         ctx->matTable.as<const float4>(), L, C, cur, shadow, objHits, plan.on ? 1 : 0,
                                          primHits);
-      rs = nomad_trace_queue(ctx, true, F.sRays.as<const float4>(), P, &C->qlen[kQ * (2)], &C->cursor[1],
+      rs = nomad_trace_queue(ctx, true, F.sRays.as<const float4>(), P, &C->qlen[kQ * shadow], &C->cursor[1],
                                nullptr, F.sOcc.as<uint8_t>(), nullptr, s);
       if (rs != NOMAD_OK) return rs;
       k_resolve<<<gridPT, kPtBlock, 0, s>>>(F.sIds.as<const uint32_t>(), F.sContrib.as<const float4>(),
-                                           F.sOcc.as<const uint8_t>(), F.rad.as<float4>(), C);
+                                           F.sOcc.as<const uint8_t>(), F.rad.as<float4>(), C, cur, shadow);
       NOMAD_CUDA(ctx, cudaGetLastError());
       cur ^= 1;
     }
