@@ -42,7 +42,8 @@ struct ViewDev {
   float cam[3], vu[3], vv[3], fp[3];
   float lod;
   uint32_t w, h, spp, maxDepth, k0, k1, flags, index;
-  uint32_t tx, ty, tw;  // the rendered tile: origin and width in the view's pixels (0, 0, w: all)
+  uint32_t tx, ty, tw, th;  // the rendered tile: origin and size in the view's pixels (0, 0, w, h: all)
+  uint32_t bw, bh;          // pixels of a camera-ray block (see queue_path); 1 x 1: row by row
   unsigned long long pathOffset, pixelOffset;
 };
 
@@ -51,6 +52,24 @@ __device__ __forceinline__ void split_path(const ViewDev &v, unsigned long long 
   const uint32_t local = (uint32_t)(pid - v.pathOffset);
   pixel = local / v.spp;
   sample = local - pixel * v.spp;
+}
+
+// The path at place i of the camera rays' queue. Paths are numbered pixel by pixel in rows; their rays
+// are queued in blocks of bw x bh pixels, about a warp's worth of paths, so that a warp's rays pass the
+// same nodes: 2.07M rays of a 1080p city view with one sample 0.377 -> 0.332 ms (8 x 4 pixels), 8.29M with
+// four 1.06 -> 1.00 (4 x 2), 921k with three 0.198 -> 0.190. Batches that are dealt out in shares of
+// less than 32 rays stay in rows (58k rays 0.057 ms, in blocks 0.060). Later bounces do not gain by it.
+__device__ __forceinline__ unsigned long long queue_path(const ViewDev &v, unsigned long long i) {
+  if (v.bh == 1) return i;
+  const uint32_t local = (uint32_t)(i - v.pathOffset);
+  const uint32_t bandPaths = v.tw * v.spp * v.bh, band = local / bandPaths;
+  const uint32_t rows = min(v.bh, v.th - band * v.bh), block = v.bw * rows * v.spp;
+  uint32_t rest = local - band * bandPaths;
+  const uint32_t col = rest / block;
+  rest -= col * block;
+  const uint32_t line = min(v.bw, v.tw - col * v.bw) * v.spp, y = rest / line;
+  rest -= y * line;  // pixels and samples into the line
+  return v.pathOffset + ((band * v.bh + y) * v.tw + col * v.bw) * v.spp + rest;
 }
 
 // The view pixel of the tile's pixel lp (row-major in the tile): the index that keys the path's
@@ -154,8 +173,9 @@ __global__ void __launch_bounds__(kPtBlock) k_raygen(const ViewDev *__restrict__
                                                       uint32_t *__restrict__ ids, float4 *__restrict__ thr,
                                                       float4 *__restrict__ rad, Counters *cnt) {
   unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long pid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; pid < P; pid += stride) {
-    const ViewDev &v = find_view(views, nviews, pid);
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < P; i += stride) {
+    const ViewDev &v = find_view(views, nviews, i);
+    const unsigned long long pid = queue_path(v, i);
     uint32_t pixel, sample;
     split_path(v, pid, pixel, sample);
     pixel = tile_pixel(v, pixel);
@@ -170,11 +190,11 @@ __global__ void __launch_bounds__(kPtBlock) k_raygen(const ViewDev *__restrict__
     V3 d = v3(v.fp[0] + s * v.vu[0] + t * v.vv[0] - v.cam[0], v.fp[1] + s * v.vu[1] + t * v.vv[1] - v.cam[1],
               v.fp[2] + s * v.vu[2] + t * v.vv[2] - v.cam[2]);
     V3 dir = normalize(d);
-    rays[2 * pid] = make_float4(v.cam[0], v.cam[1], v.cam[2], kRayEps);
-    rays[2 * pid + 1] = make_float4(dir.x, dir.y, dir.z, INFINITY);
-    ids[pid] = (uint32_t)pid;
-    thr[pid] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-    rad[pid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    rays[2 * i] = make_float4(v.cam[0], v.cam[1], v.cam[2], kRayEps);
+    rays[2 * i + 1] = make_float4(dir.x, dir.y, dir.z, INFINITY);
+    ids[i] = (uint32_t)pid;
+    thr[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    rad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     cnt->qlen[kQ * 0] = (uint32_t)P;
@@ -881,6 +901,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
       th = t.height;
     }
     d.tw = tw;
+    d.th = th;
     d.pathOffset = P;
     d.pixelOffset = pixels;
     P += (unsigned long long)tw * th * v.spp;
@@ -888,6 +909,12 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
     maxDepth = std::max(maxDepth, v.max_depth);
   }
   if (P > 0xffffffffull) return nomad_fail(ctx, NOMAD_ERR_LIMIT, "more than 2^32 paths in one frame");
+  for (ViewDev &d : vd) {
+    d.bw = d.spp == 1 ? 8 : d.spp <= 4 ? 4 : 2;
+    d.bh = d.spp <= 2 ? 4 : 2;
+    // rows where a pixel's samples fill a warp's better part, and of a view lower than a block
+    if (d.spp > 8 || P <= ctx->smCount * 28ull * 32 || d.th < d.bh) d.bw = d.bh = 1;
+  }
   FrameState &F = ctx->frame;
   nomad_status st = nomad_lights_update(ctx);
   if (st != NOMAD_OK) return st;
@@ -1230,7 +1257,7 @@ constexpr size_t kRiFixed = (kRiBlock / 32) * sizeof(RiWarp);
 
 __global__ void __launch_bounds__(kRiBlock, 1) k_restir_initial(
     const ViewDev *__restrict__ views, uint32_t nviews, unsigned long long P, RestirDev cfg,
-    const float4 *__restrict__ rays, const int32_t *__restrict__ hits,
+    const float4 *__restrict__ rays, const uint32_t *__restrict__ ids, const int32_t *__restrict__ hits,
     const ShadeTables mats, Lights L, Resv *__restrict__ rOut, Surf *__restrict__ sOut, uint32_t cdfCap,
     Counters *cnt) {
   extern __shared__ float4 riShared[];
@@ -1245,18 +1272,18 @@ __global__ void __launch_bounds__(kRiBlock, 1) k_restir_initial(
     if (lane == 0) base = atomicAdd(&cnt->riNext, 32ull);
     base = __shfl_sync(full, base, 0);
     if (base >= P) break;
-    const unsigned long long pid = base + lane;
+    const unsigned long long at = base + lane, pid = at < P ? ids[at] : P;
     Surf s;
     s.p = s.n = s.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     bool on = false;
     uint32_t pixel = 0, sample = 0, view = 0, k0 = 0, k1 = 0;
     if (pid < P) {
       const ViewDev &v = find_view(views, nviews, pid);
-      const int32_t *h = hits + 5 * pid;
+      const int32_t *h = hits + 5 * at;
       const int32_t prim = h[1];
       if ((v.flags & NOMAD_VIEW_RESTIR) && prim >= 0 && lightCount > 0 && lightTotal > 0.0f) {
         float t = __int_as_float(h[2]);
-        V3 o = ld3(rays[2 * pid]), d = ld3(rays[2 * pid + 1]);
+        V3 o = ld3(rays[2 * at]), d = ld3(rays[2 * at + 1]);
         V3 p = v3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
         V3 n = record_normal(__ldg(mats.rec + prim), p);
         if (!(dot(n, d) < 0.0f)) n = -n;
@@ -1656,7 +1683,7 @@ struct RefRing {
 
 __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
     const ViewDev *__restrict__ views, uint32_t nviews, unsigned long long P, RestirDev cfg,
-    const float4 *__restrict__ rays, const int32_t *__restrict__ hits,
+    const float4 *__restrict__ rays, const uint32_t *__restrict__ ids, const int32_t *__restrict__ hits,
     const ShadeTables mats, Lights L, Surf *__restrict__ sOut, uint32_t *__restrict__ mask, RefArgs ra,
     float4 *__restrict__ qRays, uint32_t *__restrict__ qIds, Counters *cnt, uint32_t cdfCap) {
   extern __shared__ float4 lsShared[];
@@ -1683,7 +1710,8 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   const unsigned long long iters = (P + stride - 1) / stride;
   for (unsigned long long it = 0; it < iters; ++it) {
-    const unsigned long long pid = it * stride + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long at = it * stride + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long pid = at < P ? ids[at] : P;
     Surf s;
     s.p = s.n = s.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     uint32_t pixel = 0, sample = 0;
@@ -1691,11 +1719,11 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
     if (pid < P) {
       const ViewDev &v = find_view(views, nviews, pid);
       vp = &v;
-      const int32_t *h = hits + 5 * pid;
+      const int32_t *h = hits + 5 * at;
       const int32_t prim = h[1];
       if ((v.flags & NOMAD_VIEW_RESTIR) && prim >= 0 && lightCount > 0 && lightTotal > 0.0f) {
         float t = __int_as_float(h[2]);
-        V3 o = ld3(rays[2 * pid]), d = ld3(rays[2 * pid + 1]);
+        V3 o = ld3(rays[2 * at]), d = ld3(rays[2 * at + 1]);
         V3 p = v3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
         V3 n = record_normal(__ldg(mats.rec + prim), p);
         if (!(dot(n, d) < 0.0f)) n = -n;
@@ -2010,7 +2038,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
     const ViewDev *PV = F.prevViews.as<const ViewDev>();
     k_restir_ref_reset<<<1, 1, 0, s>>>(C);
     k_restir_ref_cand<<<grid, kPtBlock, ls_bytes(cdfCap), s>>>(V, nviews, P, cfg, F.qRays[0].as<const float4>(),
-                                               F.hits.as<const int32_t>(),
+                                               F.qIds[0].as<const uint32_t>(), F.hits.as<const int32_t>(),
                                                ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, sCur, F.refMask.as<uint32_t>(), ra,
                                                F.refRays.as<float4>(), F.refIds.as<uint32_t>(), C, cdfCap);
     NOMAD_CUDA(ctx, cudaGetLastError());
@@ -2042,7 +2070,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
     return NOMAD_OK;
   }
   k_restir_initial<<<ctx->smCount, kRiBlock, kRiFixed + ls_bytes(cdfCap), s>>>(
-      V, nviews, P, cfg, F.qRays[0].as<const float4>(), F.hits.as<const int32_t>(),
+      V, nviews, P, cfg, F.qRays[0].as<const float4>(), F.qIds[0].as<const uint32_t>(), F.hits.as<const int32_t>(),
       ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, F.rInit.as<Resv>(), sCur, cdfCap, C);
   k_restir_temporal<<<grid, kPtBlock, 0, s>>>(V, F.prevViews.as<const ViewDev>(), nviews, P, cfg,
                                              ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, F.rInit.as<const Resv>(), sCur,
