@@ -9,8 +9,10 @@
 // walk's bit for bit: every record of a leaf is tested against the same ray in the same
 // arithmetic, and the order of the tests does not matter.
 //
-// What bounds it: instruction issue (77 % of active cycles on coherent rays, 71 % on diffuse
-// bounces), with the half-rate ALU pipe (min, max, compare, select) nearly full. A per-lane walk
+// What bounds it: instruction issue on coherent rays (75 % of active cycles, the half-rate pipe of
+// min, max, compare and select at 56 %), the L1's load-store wavefronts on diffuse bounces (77 % of its
+// peak: each lane reads seven rows of another node). Whole nodes in four 32-byte loads, with near and
+// far planes chosen in registers, took 1.54 ms for the bounces instead of 1.46. A per-lane walk
 // spends most of its issue slots on leaves: lanes reach them at different steps, and a loop over
 // six records runs at 4 to 9 of 32 lanes. Measured on the 2.48M-triangle city, 4-wide nodes, the
 // per-lane persistent walk before and this one: 8.29M primary rays 1.19 -> 1.06 ms, 4.98M diffuse
