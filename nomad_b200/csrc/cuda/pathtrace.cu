@@ -438,13 +438,17 @@ __device__ __forceinline__ uint32_t select_light(float xi, const Lights &L, uint
 }
 
 // select_light over a CDF staged in shared memory when it fits (cap entries), with a table of where
-// 1,024 equal steps of the CDF begin: with finite weights the CDF rises monotonically and so does a
-// draw's place in it, so a draw searches between two entries (2 to 5 steps for 4,160 lights
-// instead of 13) and finds the same slot. Built by every thread of the block.
-constexpr uint32_t kLsSteps = 1024;
-constexpr size_t kLsTable = ((kLsSteps + 1) * 2 + 14) / 16 * 16;
+// STEPS equal steps of the CDF begin: with finite weights the CDF rises monotonically and so does a
+// draw's place in it, so a draw searches between two entries (2 to 5 steps of 1,024 for 4,160 lights
+// instead of 13, 0 to 3 of 8,192) and finds the same slot. Built by every thread of the block: where one
+// block lives through the frame (k_restir_initial) the finer table pays (1080p frame 2.016 ms with
+// 1,024 steps, 1.980 with 8,192); the reference mode's kernels build it in 1,184 blocks each, and lose by it
+// (2.51 against 2.59 ms).
+constexpr uint32_t kLsFine = 8192, kLsCoarse = 1024;
 constexpr uint32_t kLsMost = 8192;  // more lights are searched in global memory
-constexpr size_t ls_bytes(uint32_t cap) { return kLsTable + (size_t)cap * sizeof(float); }
+__host__ __device__ constexpr size_t ls_table(uint32_t steps) { return ((steps + 1) * 2 + 14) / 16 * 16; }
+constexpr size_t ls_bytes(uint32_t steps, uint32_t cap) { return ls_table(steps) + (size_t)cap * sizeof(float); }
+template <uint32_t STEPS>
 struct LightSearch {
   const Lights &L;
   uint32_t count;
@@ -458,13 +462,13 @@ struct LightSearch {
     staged = count <= cap;
     stepped = staged && isfinite(total);
     step = static_cast<uint16_t *>(shared);
-    cdf = reinterpret_cast<float *>(static_cast<unsigned char *>(shared) + kLsTable);
+    cdf = reinterpret_cast<float *>(static_cast<unsigned char *>(shared) + ls_table(STEPS));
     if (staged)
       for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) cdf[i] = L.cdf[i];
     __syncthreads();
     if (stepped)
-      for (uint32_t i = threadIdx.x; i <= kLsSteps; i += blockDim.x)
-        step[i] = (uint16_t)lower((float)i * (1.0f / kLsSteps) * total, 0, count);
+      for (uint32_t i = threadIdx.x; i <= STEPS; i += blockDim.x)
+        step[i] = (uint16_t)lower((float)i * (1.0f / STEPS) * total, 0, count);
     __syncthreads();
   }
   __device__ __forceinline__ uint32_t lower(float target, uint32_t lo, uint32_t hi) const {
@@ -478,7 +482,7 @@ struct LightSearch {
   // the slot of the uniform number u01(x)
   __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
     if (!staged) return select_light(u01(x), L, count, total);
-    const uint32_t k = x >> 22;
+    const uint32_t k = x / (0x80000000u / STEPS * 2u);  // u01(x) lies in step k
     const uint32_t lo = lower(u01(x) * total, stepped ? step[k] : 0u, stepped ? step[k + 1] : count);
     return lo < count - 1 ? lo : count - 1;
   }
@@ -1262,7 +1266,7 @@ __global__ void __launch_bounds__(kRiBlock, 1) k_restir_initial(
     Counters *cnt) {
   extern __shared__ float4 riShared[];
   RiWarp &W = reinterpret_cast<RiWarp *>(riShared)[threadIdx.x >> 5];
-  const LightSearch find(L, cdfCap, reinterpret_cast<unsigned char *>(riShared) + kRiFixed);
+  const LightSearch<kLsFine> find(L, cdfCap, reinterpret_cast<unsigned char *>(riShared) + kRiFixed);
   const uint32_t lightCount = find.count;
   const float lightTotal = find.total;
   const int lane = threadIdx.x & 31;
@@ -1582,7 +1586,8 @@ __device__ __forceinline__ bool ref_geometry(const Surf &s, const BsdfView *b, V
 }
 
 // New candidate c of a path (Philox stream 0x10000 + c, as in the configuration).
-__device__ __forceinline__ bool ref_new_candidate(const Surf &s, const BsdfView *b, const Lights &L, const LightSearch &find,
+__device__ __forceinline__ bool ref_new_candidate(const Surf &s, const BsdfView *b, const Lights &L,
+                                                  const LightSearch<kLsCoarse> &find,
                                                   U4 u, RefCand &c) {
   const uint32_t off = find(u.x);
   const float4 *rec = L.rec + 5ull * off;
@@ -1688,7 +1693,7 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_cand(
     float4 *__restrict__ qRays, uint32_t *__restrict__ qIds, Counters *cnt, uint32_t cdfCap) {
   extern __shared__ float4 lsShared[];
   __shared__ RefRing rings[kPtBlock / 32];
-  const LightSearch find(L, cdfCap, lsShared);
+  const LightSearch<kLsCoarse> find(L, cdfCap, lsShared);
   RefRing &ring = rings[threadIdx.x / 32];
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
   uint32_t head = 0, done = 0;  // rays put into and written out of the warp's ring
@@ -1789,7 +1794,7 @@ __global__ void __launch_bounds__(kPtBlock, NOMAD_PT_MINB) k_restir_ref_reuse(
     int usePrev, Resv *__restrict__ rMid, float4 *__restrict__ midContrib, uint32_t *__restrict__ reuseMask,
     float4 *__restrict__ qRays, uint32_t *__restrict__ qIds, Counters *cnt, uint32_t cdfCap) {
   extern __shared__ float4 lsShared[];
-  const LightSearch find(L, cdfCap, lsShared);
+  const LightSearch<kLsCoarse> find(L, cdfCap, lsShared);
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   const unsigned long long iters = (P + stride - 1) / stride;
   for (unsigned long long it = 0; it < iters; ++it) {
@@ -2028,16 +2033,16 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
   const uint32_t cdfCap = std::min<uint32_t>(ctx->res.emissiveCount, kLsMost);  // lights staged in shared memory
   if (!F.restirSmemSet) {
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_restir_initial, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kRiFixed + ls_bytes(kLsMost))));
+                                         (int)(kRiFixed + ls_bytes(kLsFine, kLsMost))));
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_restir_ref_cand, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)ls_bytes(kLsMost)));  // beside 18 KB of rings
+                                         (int)ls_bytes(kLsCoarse, kLsMost)));  // beside 18 KB of rings
     F.restirSmemSet = true;
   }
   if (cf.reference_mode) {
     const RefArgs ra{F.lightPdf.as<const float>(), ctx->primCount, (cf.candidates + 31) / 32};
     const ViewDev *PV = F.prevViews.as<const ViewDev>();
     k_restir_ref_reset<<<1, 1, 0, s>>>(C);
-    k_restir_ref_cand<<<grid, kPtBlock, ls_bytes(cdfCap), s>>>(V, nviews, P, cfg, F.qRays[0].as<const float4>(),
+    k_restir_ref_cand<<<grid, kPtBlock, ls_bytes(kLsCoarse, cdfCap), s>>>(V, nviews, P, cfg, F.qRays[0].as<const float4>(),
                                                F.qIds[0].as<const uint32_t>(), F.hits.as<const int32_t>(),
                                                ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, sCur, F.refMask.as<uint32_t>(), ra,
                                                F.refRays.as<float4>(), F.refIds.as<uint32_t>(), C, cdfCap);
@@ -2048,7 +2053,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
     k_restir_ref_vis<<<grid, kPtBlock, 0, s>>>(F.refIds.as<const uint32_t>(), F.refOcc.as<const uint8_t>(),
                                               cf.candidates, ra.words, F.refMask.as<uint32_t>(), C);
     k_restir_ref_reset<<<1, 1, 0, s>>>(C);
-    k_restir_ref_reuse<<<grid, kPtBlock, ls_bytes(cdfCap), s>>>(V, PV, nviews, P, cfg, ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, sCur,
+    k_restir_ref_reuse<<<grid, kPtBlock, ls_bytes(kLsCoarse, cdfCap), s>>>(V, PV, nviews, P, cfg, ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, sCur,
                                                 F.refMask.as<const uint32_t>(), ra, F.resv[cur ^ 1].as<const Resv>(),
                                                 F.surf[cur ^ 1].as<const Surf>(), plan.temporal, F.rInit.as<Resv>(),
                                                 F.refContrib.as<float4>(), F.reuseMask.as<uint32_t>(),
@@ -2069,7 +2074,7 @@ nomad_status restir_launch(nomad_ctx *ctx, uint32_t nviews, unsigned long long P
     NOMAD_CUDA(ctx, cudaMemcpyAsync(F.prevViews.p, F.views.p, nviews * sizeof(ViewDev), cudaMemcpyDeviceToDevice, s));
     return NOMAD_OK;
   }
-  k_restir_initial<<<ctx->smCount, kRiBlock, kRiFixed + ls_bytes(cdfCap), s>>>(
+  k_restir_initial<<<ctx->smCount, kRiBlock, kRiFixed + ls_bytes(kLsFine, cdfCap), s>>>(
       V, nviews, P, cfg, F.qRays[0].as<const float4>(), F.qIds[0].as<const uint32_t>(), F.hits.as<const int32_t>(),
       ShadeTables{ctx->shadeRec.as<const float4>(), ctx->matTable.as<const float4>()}, L, F.rInit.as<Resv>(), sCur, cdfCap, C);
   k_restir_temporal<<<grid, kPtBlock, 0, s>>>(V, F.prevViews.as<const ViewDev>(), nviews, P, cfg,
