@@ -943,11 +943,13 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
   NOMAD_CUDA(ctx, F.views.reserve(nviews * sizeof(ViewDev)));
   cudaStream_t s = ctx->stream;
   // A frame starts when the work before it has ended, as callers that reuse the last frame's output
-  // count on. The wait stands before the view table's copy: a copy from pageable memory returns once the
-  // table is staged, so the copy itself needs none (waiting for it cost the host a round trip
+  // count on. The wait stands before the view table's copy, whose source then lives in the context until the
+  // next frame's wait, so the copy itself needs none (waiting for it cost the host a round trip
   // between every two frames: 321x181 preview 293 us a frame, 282 now).
   NOMAD_CUDA(ctx, cudaStreamSynchronize(s));
-  NOMAD_CUDA(ctx, cudaMemcpyAsync(F.views.p, vd.data(), nviews * sizeof(ViewDev), cudaMemcpyHostToDevice, s));
+  const unsigned char *table = reinterpret_cast<const unsigned char *>(vd.data());
+  F.viewTable.assign(table, table + nviews * sizeof(ViewDev));
+  NOMAD_CUDA(ctx, cudaMemcpyAsync(F.views.p, F.viewTable.data(), F.viewTable.size(), cudaMemcpyHostToDevice, s));
 
   const ViewDev *V = F.views.as<const ViewDev>();
   Counters *C = F.counters.as<Counters>();

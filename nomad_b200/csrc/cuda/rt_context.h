@@ -54,6 +54,7 @@ struct FrameState {
   DeviceBuf sOcc;                     // 1 byte per shadow entry
   DeviceBuf counters;                 // queue lengths, cursors, statistics
   DeviceBuf views;                    // view table
+  std::vector<unsigned char> viewTable;  // and the host copy that it is sent from
   DeviceBuf lightIdx, lightCdf, lightPdf, lightMeta;
   DeviceBuf lightRec;                 // 5 float4 per CDF slot, then 2 for culling (pt_lights.cuh)
   bool lightsDirty = true;
