@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS
                                                   uint64_t n, const uint32_t *__restrict__ lenDev,
                                                   unsigned long long *__restrict__ cursor,
                                                   int32_t *__restrict__ hits5, uint8_t *__restrict__ occ,
-                                                  uint32_t *__restrict__ counts, uint32_t chunk) {
+                                                  uint32_t *__restrict__ counts, uint32_t chunk, uint32_t sms) {
   const uint64_t N = lenDev ? (uint64_t)*lenDev : n;
   if constexpr (!PERSIST) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS
       store_result(hits5, i, h, counts);
   } else {
     __shared__ CoopShared sh;
+    if (lenDev && !cursor) chunk = coop_share((uint32_t)N, sms);  // the shares of the rays that are there
     coop_trace<W, STACK, ANY>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, [&](uint64_t i, const HitRec &h) {
       if (ANY)
         occ[i] = h.prim >= 0 ? 1 : 0;
@@ -593,33 +594,27 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
     constexpr uint64_t kMost = 1ull << 31;
     for (uint64_t off = 0; off < n; off += kMost) {
       const uint64_t m = lenDev ? n : std::min(kMost, n - off);
-      // A batch that gives 28 warps per SM at most 32 rays each is dealt out in equal shares, down to
-      // 8 rays: the chip has lanes to spare and a warp waits for its slowest lane (1,000 rays of a
-      // lone call: 18.5 us in 32s, 14.4 in 8s; a 58k-ray two-bounce frame 342 against 288 us).
-      // Larger ones take 32 rays at a time from the cursor. Without a cursor (the caller may run
-      // calls on several streams at once) the shares grow to 128 rays and the block scheduler deals
-      // them out, which costs 5 to 8 % (8.3M primary rays 1.11 against 1.06 ms, 4.98M bounces 1.57
+      // Batches of more than 32 rays for each of 28 warps per SM take 32 rays at a time from the cursor;
+      // without one (the caller may run calls on several streams at once) the block scheduler deals
+      // out shares, which costs 5 to 8 % (8.3M primary rays 1.11 against 1.06 ms, 4.98M bounces 1.57
       // against 1.46).
-      const uint64_t share = (m + ctx->smCount * 28ull - 1) / (ctx->smCount * 28ull);
-      uint32_t chunk = 0;
-      if (share <= 32)
-        chunk = std::max<uint32_t>(8u, ((uint32_t)share + 3u) & ~3u);
-      else if (!cursor)
-        chunk = (uint32_t)std::min<uint64_t>(128, (share + 31) & ~31ull);
-      const uint64_t warps = chunk ? (m + chunk - 1) / chunk : std::min<uint64_t>((uint64_t)ctx->smCount * perSm * (kBlock / 32), (m + 31) / 32);
+      const bool shares = !cursor || m <= ctx->smCount * 896ull;
+      const uint32_t chunk = shares ? coop_share((uint32_t)m, ctx->smCount) : 0;
+      const uint64_t warps = !shares ? std::min<uint64_t>((uint64_t)ctx->smCount * perSm * (kBlock / 32), (m + 31) / 32)
+                             : lenDev ? coop_shares((uint32_t)m, ctx->smCount) : (m + chunk - 1) / chunk;
       const uint64_t blocks = (warps + kBlock / 32 - 1) / (kBlock / 32);
       // callers with a queue on the device clear its cursor there, with the queue's length
-      if (!chunk && !lenDev) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
-      kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays + 2 * off, m, lenDev, chunk ? nullptr : cursor,
+      if (!shares && !lenDev) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
+      kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays + 2 * off, m, lenDev, shares ? nullptr : cursor,
                                                 hits5 ? hits5 + 5 * off : nullptr, occ ? occ + off : nullptr, counts,
-                                                chunk);
+                                                chunk, (uint32_t)ctx->smCount);
       NOMAD_CUDA(ctx, cudaGetLastError());
       if (lenDev) break;
     }
   } else {
     const uint64_t blocks = (n + kBlock - 1) / kBlock;
     if (blocks > 0x7fffffffull) return nomad_fail(ctx, NOMAD_ERR_LIMIT, "too many rays for one call");
-    kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays, n, lenDev, cursor, hits5, occ, counts, 0u);
+    kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays, n, lenDev, cursor, hits5, occ, counts, 0u, 0u);
     NOMAD_CUDA(ctx, cudaGetLastError());
   }
   return NOMAD_OK;
