@@ -176,9 +176,10 @@ typedef struct nomad_traversal {
   uint32_t staged_nodes;    /* persistent = 2: top-level nodes staged in shared memory         */
   uint32_t block;           /* threads per block: 0 (default 128), 64, 128, 256                */
   uint32_t postpone_leaves; /* persistent = 2: 1 = park the first leaf and keep descending     */
-  uint32_t min_blocks;      /* persistent = 0: resident blocks per SM the compiler must fit (0 =  */
-                            /* no bound; 10, 12 or 16 cap registers for occupancy); accepted and */
-                            /* without effect for persistent = 1, whose kernel has one build     */
+  uint32_t min_blocks;      /* persistent = 0 or 1: resident blocks per SM the compiler must   */
+                            /* fit (0 = no bound; 10, 12 or 16 cap registers for occupancy);   */
+                            /* without effect where persistent = 1 tests leaves cooperatively, */
+                            /* which is all but scenes of one-record leaves or < 16 primitives */
 } nomad_traversal;
 nomad_status nomad_set_traversal(nomad_ctx *ctx, const nomad_traversal *cfg);
 nomad_status nomad_get_traversal(nomad_ctx *ctx, nomad_traversal *cfg);

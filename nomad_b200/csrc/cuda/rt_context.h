@@ -103,6 +103,7 @@ struct nomad_ctx {
   nomad_traversal trav{2, 0, 0, 1, 0, 128, 0, 0};  // kernel configuration of the trace calls
   bool travAuto = true;  // the caller has not chosen one: the library picks (nomad_trace_queue)
   bool sceneReady = false;
+  float leafRecords = 0.0f;  // the scene's mean records per leaf
   // scene sizes
   uint32_t primCount = 0, objectCount = 0;
   // device memory
@@ -252,7 +253,7 @@ nomad_status nomad_patch_wide(nomad_ctx *ctx);
 nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, bool any, const float4 *rays, uint64_t n,
                                  const uint32_t *lenDev, unsigned long long *cursor, int32_t *hits5,
                                  uint8_t *occ, uint32_t *counts, cudaStream_t st);
-// The same with the context's configuration, or the library's choice where the caller made none.
+// The same trace with the context's configuration, or the library's choice where the caller made none.
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,
                                cudaStream_t st);

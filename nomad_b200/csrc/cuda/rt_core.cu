@@ -64,34 +64,46 @@ __device__ __forceinline__ void store_result(int32_t *__restrict__ hits5, uint64
   if (counts) warp_count_object_hit(h.prim >= 0 ? h.inst : -1, counts);
 }
 
-// One ray per thread (PERSIST = false) or persistent warps with cooperative leaf tests.
-template <int W, int STACK, bool ANY, bool PERSIST, int MINB>
+// One ray per thread, persistent warps whose lanes walk on their own, or persistent warps with
+// cooperative leaf tests.
+enum class Walk { PerThread, PerLane, Coop };
+
+template <int W, int STACK, bool ANY, Walk WALK, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS, const float4 *__restrict__ rays,
                                                   uint64_t n, const uint32_t *__restrict__ lenDev,
                                                   unsigned long long *__restrict__ cursor,
                                                   int32_t *__restrict__ hits5, uint8_t *__restrict__ occ,
                                                   uint32_t *__restrict__ counts, uint32_t chunk, uint32_t sms) {
   const uint64_t N = lenDev ? (uint64_t)*lenDev : n;
-  if constexpr (!PERSIST) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    float4 a = __ldg(rays + 2 * i), b = __ldg(rays + 2 * i + 1);
-    RayP r = prep_ray(a, b);
-    HitRec h;
-    trace_one<W, STACK, ANY>(S, WS, r, b.w, h);
+  auto store = [&](uint64_t i, const HitRec &h) {
     if (ANY)
       occ[i] = h.prim >= 0 ? 1 : 0;
     else
       store_result(hits5, i, h, counts);
+  };
+  auto walk = [&](uint64_t i) {
+    const float4 a = __ldg(rays + 2 * i), b = __ldg(rays + 2 * i + 1);
+    HitRec h;
+    trace_one<W, STACK, ANY>(S, WS, prep_ray(a, b), b.w, h);
+    store(i, h);
+  };
+  if constexpr (WALK == Walk::PerThread) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N) walk(i);
+  } else if constexpr (WALK == Walk::PerLane) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(cursor, 32ull);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= N) break;
+      if (base + lane < N) walk(base + lane);
+      __syncwarp();
+    }
   } else {
     __shared__ CoopShared sh;
     if (lenDev && !cursor) chunk = coop_share((uint32_t)N, sms);  // the shares of the rays that are there
-    coop_trace<W, STACK, ANY>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, [&](uint64_t i, const HitRec &h) {
-      if (ANY)
-        occ[i] = h.prim >= 0 ? 1 : 0;
-      else
-        store_result(hits5, i, h, counts);
-    });
+    coop_trace<W, STACK, ANY>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, store);
   }
 }
 
@@ -377,6 +389,15 @@ extern "C" nomad_status nomad_scene_upload(nomad_ctx *ctx, const float *bvh, uin
   S.rootRef = L.rootRef;
   S.tlasPairs = L.tlasPairCount;
   S.triCount = (int32_t)primCount;
+  {  // what the choice of a persistent walk depends on
+    uint32_t leaves = 0;
+    for (uint32_t k = 0; k < primCount; ++k) {
+      int32_t meta;
+      std::memcpy(&meta, &L.tris[12ull * k + 11], 4);
+      leaves += (meta & kLastInLeaf) != 0;
+    }
+    ctx->leafRecords = leaves ? (float)primCount / (float)leaves : 0.0f;
+  }
   S.status = static_cast<uint32_t *>(ctx->status.p);
   ctx->primCount = primCount;
   ctx->objectCount = objectCount;
@@ -581,15 +602,29 @@ namespace {
 // Stack entries of each variant: pair nodes 64; 4-wide 64; 8-wide 96.
 constexpr int kStackW4 = 64, kStackW8 = 96;
 
-template <int W, int STACK, bool ANY, bool PERSIST, int MINB>
+// Whether persistent warps walk n rays of the scene with cooperative leaf tests. Lane by lane they are
+// faster where there is nothing to share, in leaves of one record (8,192 objects of one triangle,
+// 4-wide: 60k random rays 151 us with cooperative tests against 124, 1M coherent ones 477 against 361; a
+// 1280x720 frame of three bounces 1,639 against 1,534) and in scenes of a few primitives (six triangles, 1M
+// rays: 40 us against 34; with 12 frames are within 5 %, with 60 the cooperative ones take 0.5 to 0.9 of
+// the time). With two records a leaf the tests gain as much as they lose. In batches of up
+// to a ray for each of 28 warps per SM the equal shares of the cooperative kernel decide (1,000 rays: 0.7 to
+// 1.0 of the time). What remains slower with the tests are coherent batches of about a million rays into
+// scenes of less than a few hundred primitives (250 triangles: 1.1 to 1.25; incoherent ones 0.5).
+bool coop_pays(const nomad_ctx *ctx, uint64_t n) {
+  return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) || n <= ctx->smCount * 28ull;
+}
+
+template <int W, int STACK, bool ANY, Walk WALK, int MINB>
 nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                         unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts, cudaStream_t st) {
-  auto kern = k_trace<W, STACK, ANY, PERSIST, MINB>;
-  if constexpr (PERSIST) {
-    static const int perSm = [kern] {  // resident blocks per SM, of every sm_100 device
-      int k = 0;
-      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kBlock, 0) == cudaSuccess && k > 0 ? k : 1;
-    }();
+  auto kern = k_trace<W, STACK, ANY, WALK, MINB>;
+  static const int perSm = [kern] {  // resident blocks per SM, of every sm_100 device
+    int k = 0;
+    return WALK != Walk::PerThread &&
+                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kBlock, 0) == cudaSuccess && k > 0 ? k : 1;
+  }();
+  if constexpr (WALK == Walk::Coop) {
     // ray indices are 32 bits in the kernel; a queue's length on the device is 32 bits already
     constexpr uint64_t kMost = 1ull << 31;
     for (uint64_t off = 0; off < n; off += kMost) {
@@ -612,7 +647,11 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
       if (lenDev) break;
     }
   } else {
-    const uint64_t blocks = (n + kBlock - 1) / kBlock;
+    uint64_t blocks = (n + kBlock - 1) / kBlock;
+    if (WALK == Walk::PerLane) {
+      blocks = std::min<uint64_t>((uint64_t)ctx->smCount * perSm, blocks);
+      if (!lenDev) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
+    }
     if (blocks > 0x7fffffffull) return nomad_fail(ctx, NOMAD_ERR_LIMIT, "too many rays for one call");
     kern<<<(unsigned)blocks, kBlock, 0, st>>>(ctx->scene, WS, rays, n, lenDev, cursor, hits5, occ, counts, 0u, 0u);
     NOMAD_CUDA(ctx, cudaGetLastError());
@@ -620,37 +659,39 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
   return NOMAD_OK;
 }
 
-template <int W, int STACK, bool ANY, bool PERSIST>
+template <int W, int STACK, bool ANY, Walk WALK>
 nomad_status launch_minb(nomad_ctx *ctx, uint32_t minBlocks, const WideScene &WS, const float4 *rays, uint64_t n,
                          const uint32_t *lenDev, unsigned long long *cursor, int32_t *hits5, uint8_t *occ,
                          uint32_t *counts, cudaStream_t st) {
-  if (minBlocks != 0 && minBlocks != 10 && minBlocks != 12 && minBlocks != 16)
-    return nomad_fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "min_blocks must be 0, 10, 12 or 16");
-  if constexpr (PERSIST) {  // one build, at the occupancy that was measured best
-    return launch_one<W, STACK, ANY, true, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-  } else {
-    switch (minBlocks) {
-      case 0: return launch_one<W, STACK, ANY, false, 1>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-      case 10: return launch_one<W, STACK, ANY, false, 10>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-      case 12: return launch_one<W, STACK, ANY, false, 12>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-      default: return launch_one<W, STACK, ANY, false, 16>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    }
+  switch (minBlocks) {
+    case 0: return launch_one<W, STACK, ANY, WALK, 1>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 10: return launch_one<W, STACK, ANY, WALK, 10>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 12: return launch_one<W, STACK, ANY, WALK, 12>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 16: return launch_one<W, STACK, ANY, WALK, 16>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    default: return nomad_fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "min_blocks must be 0, 10, 12 or 16");
   }
+}
+
+template <int W, int STACK, bool ANY>
+nomad_status launch_walk(nomad_ctx *ctx, const nomad_traversal &c, const WideScene &WS, const float4 *rays, uint64_t n,
+                         const uint32_t *lenDev, unsigned long long *cursor, int32_t *hits5, uint8_t *occ,
+                         uint32_t *counts, cudaStream_t st) {
+  if (c.persistent == 0)
+    return launch_minb<W, STACK, ANY, Walk::PerThread>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  if (cursor && !coop_pays(ctx, n))
+    return launch_minb<W, STACK, ANY, Walk::PerLane>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  // one build, at the occupancy that was measured best
+  return launch_one<W, STACK, ANY, Walk::Coop, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
 }
 
 template <bool ANY>
 nomad_status dispatch(nomad_ctx *ctx, const nomad_traversal &c, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                       unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts, cudaStream_t st) {
   const WideScene none{nullptr, kEmptyRef};
-  const bool p = c.persistent != 0;
-  const uint32_t mb = c.min_blocks;
   switch (c.width) {
-    case 2: return p ? launch_minb<2, kStack, ANY, true>(ctx, mb, none, rays, n, lenDev, cursor, hits5, occ, counts, st)
-                     : launch_minb<2, kStack, ANY, false>(ctx, mb, none, rays, n, lenDev, cursor, hits5, occ, counts, st);
-    case 4: return p ? launch_minb<4, kStackW4, ANY, true>(ctx, mb, ctx->ws[0], rays, n, lenDev, cursor, hits5, occ, counts, st)
-                     : launch_minb<4, kStackW4, ANY, false>(ctx, mb, ctx->ws[0], rays, n, lenDev, cursor, hits5, occ, counts, st);
-    case 8: return p ? launch_minb<8, kStackW8, ANY, true>(ctx, mb, ctx->ws[1], rays, n, lenDev, cursor, hits5, occ, counts, st)
-                     : launch_minb<8, kStackW8, ANY, false>(ctx, mb, ctx->ws[1], rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 2: return launch_walk<2, kStack, ANY>(ctx, c, none, rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 4: return launch_walk<4, kStackW4, ANY>(ctx, c, ctx->ws[0], rays, n, lenDev, cursor, hits5, occ, counts, st);
+    case 8: return launch_walk<8, kStackW8, ANY>(ctx, c, ctx->ws[1], rays, n, lenDev, cursor, hits5, occ, counts, st);
     default: return nomad_fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "unknown kernel variant");
   }
 }
@@ -674,21 +715,23 @@ nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, boo
 // The configuration that serves a context whose caller has not chosen one: the cooperative kernel
 // over 4-wide nodes (2.2 times the per-thread binary walk's speed on a 58k-ray frame, 1.3 to 1.7 on
 // millions of rays), or another width where that layout is not on the device or would need a
-// deeper stack.
-static nomad_traversal auto_traversal(const nomad_ctx *ctx) {
-  for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
-    const nomad_traversal c = nomad_kernel_config(k);
-    if (nomad_traversal_ok(ctx, c, nullptr)) return c;
-  }
+// deeper stack. Where it does not pay, the per-thread binary walk, unless only a wider layout is on
+// the device (paging).
+static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n) {
+  if (coop_pays(ctx, n) || ctx->trav.persistent != 0)
+    for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
+      const nomad_traversal c = nomad_kernel_config(k);
+      if (nomad_traversal_ok(ctx, c, nullptr)) return c;
+    }
   return ctx->trav;
 }
 
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,
                                cudaStream_t st) {
-  // an unchosen configuration keeps no state between launches, so calls may overlap on streams
+  // an unchosen configuration keeps no state between launches (no cursor), so calls may overlap on streams
   return ctx->travAuto
-             ? nomad_trace_variant(ctx, auto_traversal(ctx), any, rays, n, lenDev, nullptr, hits5, occ, counts, st)
+             ? nomad_trace_variant(ctx, auto_traversal(ctx, n), any, rays, n, lenDev, nullptr, hits5, occ, counts, st)
              : nomad_trace_variant(ctx, ctx->trav, any, rays, n, lenDev, cursor, hits5, occ, counts, st);
 }
 

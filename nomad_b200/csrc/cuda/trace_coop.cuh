@@ -8,6 +8,7 @@
 // finds a hit keeps the lexicographically smallest (t, primitive). The hits are the per-lane
 // walk's bit for bit: every record of a leaf is tested against the same ray in the same
 // arithmetic, and the order of the tests does not matter.
+// Scenes and batches that gain nothing by it keep a per-lane walk (coop_pays).
 //
 // What bounds it: instruction issue on coherent rays (75 % of active cycles, the half-rate pipe of
 // min, max, compare and select at 56 %), the L1's load-store wavefronts on diffuse bounces (77 % of its
