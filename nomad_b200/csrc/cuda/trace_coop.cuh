@@ -52,7 +52,7 @@ struct CoopShared {
   float4 o[kCoopBlock];   // origin; distance of the closest hit so far (tmax before)
   float4 d[kCoopBlock];   // direction; bits of the closest hit's primitive (INT32_MIN before)
   float4 hit[kCoopBlock]; // its u, v and the bits of its instance
-  uint32_t next[kCoopBlock / 32], left[kCoopBlock / 32];  // a warp's share of the batch not handed out yet
+  uint32_t next[kCoopBlock / 32], end[kCoopBlock / 32];  // a warp's rays of the batch not handed out yet
   int2 leaf[kCoopBlock];  // pending leaves of a warp: first record, lane of the ray
   int win[kCoopBlock];    // per ray: the lane whose hit is taken in this round
 };
@@ -181,13 +181,14 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
   int32_t ref = kEmptyRef;
   uint32_t ray = kNoRay;  // the lane's ray, until its result is stored
   bool more = true, mixed = false;
+  // The share is kept as its two ends: with its length, min(chunk, N - first), one build of this kernel took
+  // the whole chunk of the last share (CUDA 12.9), 7 rays beyond the batch.
+  const uint64_t first = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (wb >> 5)) * chunk;
+  if (!cursor && first >= N) return;
   if (lane == 0) {
-    const uint64_t first = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (wb >> 5)) * chunk;
-    sh.next[wb >> 5] = (uint32_t)first;
-    sh.left[wb >> 5] = cursor || first >= N ? 0u : min(chunk, N - (uint32_t)first);
+    sh.next[wb >> 5] = cursor ? N : (uint32_t)first;
+    sh.end[wb >> 5] = (uint32_t)min(first + chunk, (uint64_t)N);
   }
-  __syncwarp();
-  if (!cursor && sh.left[wb >> 5] == 0) return;
   for (;;) {
     while (ref == kEmptyRef && sp > 0) {  // the newest entry that still starts before the bound
       const StackEntry<ANY> e = stk[--sp];
@@ -242,8 +243,8 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
       }
       __syncwarp();
       if (!more) break;  // nothing busy and nothing left
-      uint32_t next = sh.next[wb >> 5], left = sh.left[wb >> 5];
-      if (left == 0) {
+      uint32_t next = sh.next[wb >> 5], end = sh.end[wb >> 5];
+      if (next >= end) {
         unsigned long long base = N;
         if (cursor) {
           if (lane == 0) base = atomicAdd(cursor, 32ull);
@@ -254,10 +255,10 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
           continue;
         }
         next = (uint32_t)base;
-        left = min(32u, N - next);
+        end = N - next < 32u ? N : next + 32u;
       }
       const uint32_t rank = __popc(~busy & lt);
-      if (idle && rank < left) {
+      if (idle && rank < end - next) {
         ray = next + rank;
         const float4 a = __ldg(rays + 2ull * ray), b = __ldg(rays + 2ull * ray + 1);
         const RayP p = prep_ray(a, b);
@@ -274,11 +275,10 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
         sh.o[tid] = make_float4(a.x, a.y, a.z, b.w);
         sh.d[tid] = make_float4(b.x, b.y, b.z, __int_as_float(INT32_MIN));
       }
-      const uint32_t take = min((uint32_t)__popc(~busy), left);
       __syncwarp();
       if (lane == 0) {
-        sh.next[wb >> 5] = next + take;
-        sh.left[wb >> 5] = left - take;
+        sh.next[wb >> 5] = min(next + __popc(~busy), end);
+        sh.end[wb >> 5] = end;
       }
       // rays of one octant stay together well; mixed ones are worth refilling lane by lane
       const bool on = ray != kNoRay;
