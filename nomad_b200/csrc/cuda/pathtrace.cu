@@ -1033,6 +1033,7 @@ static nomad_status render_views(nomad_ctx *ctx, const nomad_view *views, const 
     key_put(key, ctx->trav);
     key_put(key, ctx->travAuto);
     key_put(key, ctx->leafRecords);
+    key_put(key, ctx->mostlyTris);
     key_put(key, ctx->scene);
     for (const WideScene &w : ctx->ws) {
       key_put(key, w.wn);

@@ -104,6 +104,7 @@ struct nomad_ctx {
   bool travAuto = true;  // the caller has not chosen one: the library picks (nomad_trace_queue)
   bool sceneReady = false;
   float leafRecords = 0.0f;  // the scene's mean records per leaf
+  bool mostlyTris = true;    // at least half of its primitives are triangles
   // scene sizes
   uint32_t primCount = 0, objectCount = 0;
   // device memory

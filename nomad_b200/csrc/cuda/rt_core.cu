@@ -65,8 +65,8 @@ __device__ __forceinline__ void store_result(int32_t *__restrict__ hits5, uint64
 }
 
 // One ray per thread, persistent warps whose lanes walk on their own, or persistent warps with
-// cooperative leaf tests.
-enum class Walk { PerThread, PerLane, Coop };
+// cooperative leaf tests, for scenes of mostly triangles or of mostly other primitives.
+enum class Walk { PerThread, PerLane, Coop, CoopOther };
 
 template <int W, int STACK, bool ANY, Walk WALK, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS, const float4 *__restrict__ rays,
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS
   } else {
     __shared__ CoopShared sh;
     if (lenDev && !cursor) chunk = coop_share((uint32_t)N, sms);  // the shares of the rays that are there
-    coop_trace<W, STACK, ANY>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, store);
+    coop_trace<W, STACK, ANY, WALK == Walk::CoopOther>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, store);
   }
 }
 
@@ -390,13 +390,15 @@ extern "C" nomad_status nomad_scene_upload(nomad_ctx *ctx, const float *bvh, uin
   S.tlasPairs = L.tlasPairCount;
   S.triCount = (int32_t)primCount;
   {  // what the choice of a persistent walk depends on
-    uint32_t leaves = 0;
+    uint32_t leaves = 0, tris = 0;
     for (uint32_t k = 0; k < primCount; ++k) {
       int32_t meta;
       std::memcpy(&meta, &L.tris[12ull * k + 11], 4);
       leaves += (meta & kLastInLeaf) != 0;
+      tris += (meta & 0xff) == 1;
     }
     ctx->leafRecords = leaves ? (float)primCount / (float)leaves : 0.0f;
+    ctx->mostlyTris = 2ull * tris >= primCount;
   }
   S.status = static_cast<uint32_t *>(ctx->status.p);
   ctx->primCount = primCount;
@@ -624,7 +626,7 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
     return WALK != Walk::PerThread &&
                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kBlock, 0) == cudaSuccess && k > 0 ? k : 1;
   }();
-  if constexpr (WALK == Walk::Coop) {
+  if constexpr (WALK == Walk::Coop || WALK == Walk::CoopOther) {
     // ray indices are 32 bits in the kernel; a queue's length on the device is 32 bits already
     constexpr uint64_t kMost = 1ull << 31;
     for (uint64_t off = 0; off < n; off += kMost) {
@@ -680,8 +682,10 @@ nomad_status launch_walk(nomad_ctx *ctx, const nomad_traversal &c, const WideSce
     return launch_minb<W, STACK, ANY, Walk::PerThread>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
   if (cursor && !coop_pays(ctx, n))
     return launch_minb<W, STACK, ANY, Walk::PerLane>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-  // one build, at the occupancy that was measured best
-  return launch_one<W, STACK, ANY, Walk::Coop, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  // one build each, at the occupancy that was measured best
+  return ctx->mostlyTris
+             ? launch_one<W, STACK, ANY, Walk::Coop, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st)
+             : launch_one<W, STACK, ANY, Walk::CoopOther, kCoopMinBlocks>(ctx, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
 }
 
 template <bool ANY>

@@ -139,6 +139,25 @@ __device__ __forceinline__ bool intersect_tri(float4 o, float4 d, float4 A, floa
   return (fabsf(a) > 1e-5f) & (u >= 0.0f) & (u <= 1.0f) & (v >= 0.0f) & (u + v <= 1.0f) & (tt > kRayEps);
 }
 
+// One pair of ray and record. With OTHER a record runs its own type's test alone; without, every lane
+// runs the triangles' and the few other records add theirs. Spheres and rectangles pay for the triangle
+// test that way (500 spheres, 1M coherent rays: 156 us, 119 with OTHER; a 1080p frame of 1,000 spheres
+// 5,189, 4,492), triangles for the branch the other way (city bounces 3 to 8 %).
+template <bool OTHER>
+__device__ __forceinline__ bool coop_intersect(const DevScene &S, float4 o, float4 d, float4 A, float4 B, float4 C,
+                                               int32_t pid, int type, float best, float &tt, float &u, float &v) {
+  if constexpr (!OTHER) {
+    bool hit = intersect_tri(o, d, A, B, C, tt, u, v) & (type == 1);
+    if (type != 1 && pid >= 0)
+      hit = intersect_prim(S, o.x, o.y, o.z, d.x, d.y, d.z, A, B, C, pid, type, best, tt, u, v);
+    return hit;
+  } else {
+    tt = u = v = 0.0f;
+    if (type == 1) return intersect_tri(o, d, A, B, C, tt, u, v);
+    return pid >= 0 && intersect_prim(S, o.x, o.y, o.z, d.x, d.y, d.z, A, B, C, pid, type, best, tt, u, v);
+  }
+}
+
 // Rays of a warp's share where n rays are dealt out in shares, on `sms` SMs. Up to 32 rays for each of 28
 // warps per SM: equal shares, down to 8 rays, as the chip has lanes to spare and a warp waits for
 // its slowest lane (1,000 rays of a lone call: 18.5 us in 32s, 14.4 in 8s; a 58k-ray two-bounce frame 342
@@ -165,8 +184,8 @@ __host__ __device__ constexpr uint32_t coop_shares(uint32_t n, uint32_t sms) {
 
 // Walks the rays of the batch (N < 2^32): the warp's own share of `chunk` rays, or, with a cursor, 32
 // rays at a time from it; DONE(i, h) stores the result of ray i (called by the lanes
-// that finished one, warp-divergent).
-template <int W, int STACK, bool ANY, typename DONE>
+// that finished one, warp-divergent). OTHER: most records are no triangles.
+template <int W, int STACK, bool ANY, bool OTHER, typename DONE>
 __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &WS, CoopShared &sh,
                                            const float4 *__restrict__ rays, uint32_t N, uint32_t chunk,
                                            unsigned long long *__restrict__ cursor, DONE done) {
@@ -301,9 +320,7 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
           const float4 A = ldg4(q), B = ldg4(q + 1), C = ldg4(q + 2);
           const int32_t pid = __float_as_int(A.w), meta = __float_as_int(C.w);
           float tt, u, v;
-          bool hit = intersect_tri(o, d, A, B, C, tt, u, v) & ((meta & 0xff) == 1);
-          if ((meta & 0xff) != 1 && pid >= 0)
-            hit = intersect_prim(S, o.x, o.y, o.z, d.x, d.y, d.z, A, B, C, pid, meta & 0xff, ht, tt, u, v);
+          const bool hit = coop_intersect<OTHER>(S, o, d, A, B, C, pid, meta & 0xff, ht, tt, u, v);
           if (hit & (pid >= 0) & ((tt < ht) | ((tt == ht) & (pid < hp)))) {
             ht = tt;
             hp = pid;
@@ -341,9 +358,7 @@ __device__ __forceinline__ void coop_trace(const DevScene &S, const WideScene &W
         const unsigned last = __ballot_sync(kFull, (meta & kLastInLeaf) != 0);
         const unsigned before = ((last >> (lane & 24)) & 0xffu) & ((1u << k) - 1u);  // the leaf ended earlier
         float tt, u, v;
-        bool hit = intersect_tri(o, d, A, B, C, tt, u, v) & ((meta & 0xff) == 1);
-        if ((meta & 0xff) != 1 && pid >= 0)
-          hit = intersect_prim(S, o.x, o.y, o.z, d.x, d.y, d.z, A, B, C, pid, meta & 0xff, o.w, tt, u, v);
+        bool hit = coop_intersect<OTHER>(S, o, d, A, B, C, pid, meta & 0xff, o.w, tt, u, v);
         hit = hit & (g < total) & (before == 0) & (pid >= 0) & (tt <= o.w);
         if (ANY) {
           const unsigned occ = __reduce_or_sync(kFull, hit && tt < o.w ? 1u << e.y : 0u);
