@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_trace(DevScene S, WideScene WS
     }
   } else {
     __shared__ CoopShared sh;
-    if (lenDev && !cursor) chunk = coop_share((uint32_t)N, sms);  // the shares of the rays that are there
+    if (!cursor && !chunk) chunk = coop_queue_share((uint32_t)N, sms);
     coop_trace<W, STACK, ANY, WALK == Walk::CoopOther>(S, WS, sh, rays, (uint32_t)N, chunk, cursor, store);
   }
 }
@@ -636,9 +636,12 @@ nomad_status launch_one(nomad_ctx *ctx, const WideScene &WS, const float4 *rays,
       // out shares, which costs 5 to 8 % (8.3M primary rays 1.11 against 1.06 ms, 4.98M bounces 1.57
       // against 1.46).
       const bool shares = !cursor || m <= ctx->smCount * 896ull;
-      const uint32_t chunk = shares ? coop_share((uint32_t)m, ctx->smCount) : 0;
-      const uint64_t warps = !shares ? std::min<uint64_t>((uint64_t)ctx->smCount * perSm * (kBlock / 32), (m + 31) / 32)
-                             : lenDev ? coop_shares((uint32_t)m, ctx->smCount) : (m + chunk - 1) / chunk;
+      // A small queue's share follows from its capacity (taking it from the length costs each launch more
+      // than it gives: a 48k-path frame of three bounces 384 us against 376), a larger one's from the length.
+      const uint32_t chunk = shares && (!lenDev || m <= ctx->smCount * 896ull) ? coop_share((uint32_t)m, ctx->smCount) : 0;
+      const uint64_t warps = chunk    ? (m + chunk - 1) / chunk
+                             : shares ? (m + 31) / 32  // as many as any length up to m needs
+                                      : std::min<uint64_t>((uint64_t)ctx->smCount * perSm * (kBlock / 32), (m + 31) / 32);
       const uint64_t blocks = (warps + kBlock / 32 - 1) / (kBlock / 32);
       // callers with a queue on the device clear its cursor there, with the queue's length
       if (!shares && !lenDev) NOMAD_CUDA(ctx, cudaMemsetAsync(cursor, 0, 8, st));
@@ -733,10 +736,14 @@ static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n) {
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,
                                cudaStream_t st) {
-  // an unchosen configuration keeps no state between launches (no cursor), so calls may overlap on streams
-  return ctx->travAuto
-             ? nomad_trace_variant(ctx, auto_traversal(ctx, n), any, rays, n, lenDev, nullptr, hits5, occ, counts, st)
-             : nomad_trace_variant(ctx, ctx->trav, any, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  if (!ctx->travAuto) return nomad_trace_variant(ctx, ctx->trav, any, rays, n, lenDev, cursor, hits5, occ, counts, st);
+  // An unchosen configuration keeps no state between the launches of trace calls (no cursor), so they may
+  // overlap on streams. A frame's queues belong to one frame at a time: large ones are fed from the cursor
+  // (two bounces of 3.7M paths, 82k triangles: 408 us, 447 in shares), those of up to eight rounds of 32-ray
+  // shares are not (six bounces of 921,600 paths, 117k triangles: 915 us, 1,119 from the cursor).
+  const bool feed = lenDev && n > ctx->smCount * 9216ull;
+  return nomad_trace_variant(ctx, auto_traversal(ctx, n), any, rays, n, lenDev, feed ? cursor : nullptr, hits5, occ, counts,
+                             st);
 }
 
 extern "C" nomad_status nomad_set_kernel(nomad_ctx *ctx, uint32_t kernel) {

@@ -161,25 +161,19 @@ __device__ __forceinline__ bool coop_intersect(const DevScene &S, float4 o, floa
 // Rays of a warp's share where n rays are dealt out in shares, on `sms` SMs. Up to 32 rays for each of 28
 // warps per SM: equal shares, down to 8 rays, as the chip has lanes to spare and a warp waits for
 // its slowest lane (1,000 rays of a lone call: 18.5 us in 32s, 14.4 in 8s; a 58k-ray two-bounce frame 342
-// against 288 us). Above that 32 to 128 rays: eight rounds of the 36 resident warps or more, so that the
-// last one is short. A queue's share follows from the length it has, not from its capacity: a path
-// tracer's later bounces are a fraction of it (1280x720, one sample, six bounces of an untuned
-// context in the 117k-triangle city: 1,838 us with shares of the capacity, 915 now).
+// against 288 us). Above that up to 128: coherent rays want less (1M into the 117k-triangle city: 237 us,
+// 220 in 32s), incoherent ones more, from which idle lanes are refilled (1M shadow rays there: 177 us, 204
+// in 96s).
 __host__ __device__ constexpr uint32_t coop_share(uint32_t n, uint32_t sms) {
-  const uint32_t few = n / (sms * 28) + (n % (sms * 28) != 0), some = n / (sms * 288) + (n % (sms * 288) != 0);
-  if (few <= 32) return few <= 8 ? 8u : (few + 3u) & ~3u;
-  return some >= 128 ? 128u : (some + 31u) & ~31u;
+  const uint32_t share = n / (sms * 28) + (n % (sms * 28) != 0);
+  return share <= 8 ? 8u : share <= 32 ? (share + 3u) & ~3u : share < 128 ? (share + 31u) & ~31u : 128u;
 }
 
-// The most shares that any n rays or fewer are dealt out in.
-__host__ __device__ constexpr uint32_t coop_shares(uint32_t n, uint32_t sms) {
-  uint32_t most = n / 8 < sms * 28 ? n / 8 + 1 : sms * 28;
-  if (n > sms * 896) {
-    const uint32_t mid = n / 32 < sms * 288 ? n / 32 + 1 : sms * 288, top = n / 128 + 1;
-    most = most > mid ? most : mid;
-    most = most > top ? most : top;
-  }
-  return most;
+// The same for a path tracer's queue, n the length that it has: its capacity says little, as later bounces
+// are a fraction of it (1280x720, one sample, six bounces of an untuned context in the 117k-triangle
+// city: 1,838 us with shares of the capacity, 915 now).
+__host__ __device__ constexpr uint32_t coop_queue_share(uint32_t n, uint32_t sms) {
+  return n <= sms * 896 ? coop_share(n, sms) : 32u;
 }
 
 // Walks the rays of the batch (N < 2^32): the warp's own share of `chunk` rays, or, with a cursor, 32
