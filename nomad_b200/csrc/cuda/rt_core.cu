@@ -611,10 +611,12 @@ constexpr int kStackW4 = 64, kStackW8 = 96;
 // rays: 40 us against 34; with 12 frames are within 5 %, with 60 the cooperative ones take 0.5 to 0.9 of
 // the time). With two records a leaf the tests gain as much as they lose. In batches of up
 // to a ray for each of 28 warps per SM the equal shares of the cooperative kernel decide (1,000 rays: 0.7 to
-// 1.0 of the time). What remains slower with the tests are coherent batches of about a million rays into
-// scenes of less than a few hundred primitives (250 triangles: 1.1 to 1.25; incoherent ones 0.5).
-bool coop_pays(const nomad_ctx *ctx, uint64_t n) {
-  return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) || n <= ctx->smCount * 28ull;
+// 1.0 of the time), in a frame's queues, which shrink from bounce to bounce, up to 32 rays (57,600 paths
+// of two bounces: 467 us with the tests, 519 without). What remains slower with the tests are coherent
+// batches of about a million rays into scenes of less than a few hundred primitives (250 triangles: 1.1 to
+// 1.25; incoherent ones 0.5).
+bool coop_pays(const nomad_ctx *ctx, uint64_t n, bool queue) {
+  return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) || n <= ctx->smCount * (queue ? 896ull : 28ull);
 }
 
 template <int W, int STACK, bool ANY, Walk WALK, int MINB>
@@ -683,7 +685,7 @@ nomad_status launch_walk(nomad_ctx *ctx, const nomad_traversal &c, const WideSce
                          uint32_t *counts, cudaStream_t st) {
   if (c.persistent == 0)
     return launch_minb<W, STACK, ANY, Walk::PerThread>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-  if (cursor && !coop_pays(ctx, n))
+  if (cursor && !coop_pays(ctx, n, lenDev != nullptr))
     return launch_minb<W, STACK, ANY, Walk::PerLane>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
   // one build each, at the occupancy that was measured best
   return ctx->mostlyTris
@@ -724,8 +726,8 @@ nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, boo
 // millions of rays), or another width where that layout is not on the device or would need a
 // deeper stack. Where it does not pay, the per-thread binary walk, unless only a wider layout is on
 // the device (paging).
-static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n) {
-  if (coop_pays(ctx, n) || ctx->trav.persistent != 0)
+static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n, bool queue) {
+  if (coop_pays(ctx, n, queue) || ctx->trav.persistent != 0)
     for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
       const nomad_traversal c = nomad_kernel_config(k);
       if (nomad_traversal_ok(ctx, c, nullptr)) return c;
@@ -742,7 +744,7 @@ nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uin
   // (two bounces of 3.7M paths, 82k triangles: 408 us, 447 in shares), those of up to eight rounds of 32-ray
   // shares are not (six bounces of 921,600 paths, 117k triangles: 915 us, 1,119 from the cursor).
   const bool feed = lenDev && n > ctx->smCount * 9216ull;
-  return nomad_trace_variant(ctx, auto_traversal(ctx, n), any, rays, n, lenDev, feed ? cursor : nullptr, hits5, occ, counts,
+  return nomad_trace_variant(ctx, auto_traversal(ctx, n, lenDev != nullptr), any, rays, n, lenDev, feed ? cursor : nullptr, hits5, occ, counts,
                              st);
 }
 
