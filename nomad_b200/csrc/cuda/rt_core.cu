@@ -726,13 +726,17 @@ nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, boo
 // millions of rays), or another width where that layout is not on the device or would need a
 // deeper stack. Where it does not pay, the per-thread binary walk, unless only a wider layout is on
 // the device (paging).
+static bool coop_traversal(const nomad_ctx *ctx, nomad_traversal *c) {
+  for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
+    *c = nomad_kernel_config(k);
+    if (nomad_traversal_ok(ctx, *c, nullptr)) return true;
+  }
+  return false;
+}
+
 static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n, bool queue) {
-  if (coop_pays(ctx, n, queue) || ctx->trav.persistent != 0)
-    for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
-      const nomad_traversal c = nomad_kernel_config(k);
-      if (nomad_traversal_ok(ctx, c, nullptr)) return c;
-    }
-  return ctx->trav;
+  nomad_traversal c;
+  return (coop_pays(ctx, n, queue) || ctx->trav.persistent != 0) && coop_traversal(ctx, &c) ? c : ctx->trav;
 }
 
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
@@ -753,9 +757,11 @@ extern "C" nomad_status nomad_set_kernel(nomad_ctx *ctx, uint32_t kernel) {
   const bool automatic = kernel == NOMAD_KERNEL_AUTO;
   if (automatic) kernel = NOMAD_KERNEL_BVH2;
   if (kernel >= NOMAD_KERNEL_COUNT) return fail(ctx, NOMAD_ERR_INVALID_ARGUMENT, "unknown kernel");
-  const nomad_traversal c = nomad_kernel_config(kernel);
-  if (ctx->sceneReady && !nomad_traversal_ok(ctx, c, nullptr))
-    return fail(ctx, NOMAD_ERR_UNSUPPORTED, "kernel variant needs a deeper stack than it has for this scene");
+  nomad_traversal c = nomad_kernel_config(kernel);
+  std::string why;
+  // the library's choice needs only one layout on the device (a paged scene has one)
+  if (!nomad_traversal_ok(ctx, c, &why) && !(automatic && coop_traversal(ctx, &c)))
+    return fail(ctx, NOMAD_ERR_UNSUPPORTED, why);
   ctx->trav = c;
   ctx->travAuto = automatic;
   return NOMAD_OK;
