@@ -146,8 +146,12 @@ nomad_status nomad_autotune(nomad_ctx *ctx, const nomad_ray *rays, uint64_t n, u
                             uint32_t flags, nomad_tune_result *out);
 
 /* Chooses the traversal variant used by the trace calls (NOMAD_KERNEL_*). Until one is chosen, and
- * with NOMAD_KERNEL_AUTO, the library picks per scene (nomad_get_traversal then reports the binary
- * per-thread walk) and calls on one context may overlap on several streams. */
+ * with NOMAD_KERNEL_AUTO, the library picks per scene and batch, and trace calls on one context may
+ * overlap on several streams. nomad_get_traversal then reports the binary per-thread walk, or the
+ * walk of a paged layout, with regroup = NOMAD_REGROUP_AUTO; nomad_set_traversal with the former
+ * leaves the choice to the library on that context too, and reads that regroup as 1 in any other
+ * configuration. */
+#define NOMAD_REGROUP_AUTO 0xffffffffu
 nomad_status nomad_set_kernel(nomad_ctx *ctx, uint32_t kernel);
 
 /* Full traversal configuration (no counterpart in the reference, which has one kernel). The

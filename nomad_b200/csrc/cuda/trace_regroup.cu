@@ -596,17 +596,24 @@ extern "C" nomad_status nomad_selftest_bounded_wait(nomad_ctx *ctx, int32_t comp
 
 extern "C" nomad_status nomad_set_traversal(nomad_ctx *ctx, const nomad_traversal *cfg) {
   if (!ctx || !cfg) return NOMAD_ERR_INVALID_ARGUMENT;
+  nomad_traversal c = *cfg;
+  if (!c.block) c.block = 128;
+  if (c.regroup == NOMAD_REGROUP_AUTO) {
+    c.regroup = 1;
+    const nomad_traversal unchosen = nomad_kernel_config(NOMAD_KERNEL_BVH2);
+    if (std::memcmp(&c, &unchosen, sizeof(c)) == 0) return nomad_set_kernel(ctx, NOMAD_KERNEL_AUTO);
+  }
   std::string why;
-  if (!nomad_traversal_ok(ctx, *cfg, &why)) return nomad_fail(ctx, NOMAD_ERR_UNSUPPORTED, why);
-  ctx->trav = *cfg;
+  if (!nomad_traversal_ok(ctx, c, &why)) return nomad_fail(ctx, NOMAD_ERR_UNSUPPORTED, why);
+  ctx->trav = c;
   ctx->travAuto = false;
-  if (!ctx->trav.block) ctx->trav.block = 128;
   return NOMAD_OK;
 }
 
 extern "C" nomad_status nomad_get_traversal(nomad_ctx *ctx, nomad_traversal *cfg) {
   if (!ctx || !cfg) return NOMAD_ERR_INVALID_ARGUMENT;
   *cfg = ctx->trav;
+  if (ctx->travAuto) cfg->regroup = NOMAD_REGROUP_AUTO;
   return NOMAD_OK;
 }
 

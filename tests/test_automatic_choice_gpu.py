@@ -1,5 +1,5 @@
 """GPU test of the library's own choice of a traversal: it can be taken up again on a context whose only node layout
-is a paged wide one."""
+is a paged wide one, and it goes with a configuration that is read from one context and set on another."""
 import numpy as np
 import pytest
 
@@ -31,3 +31,26 @@ def test_automatic_again_while_paging(nb, small_city, width):
         assert ctx.status() == 0
     finally:
         ctx.close()
+
+
+def test_unchosen_configuration_goes_with_the_dict(nb, small_city):
+    sb = small_city[1]
+    a, b = nb.Context(0), nb.Context(0)
+    try:
+        for c in (a, b):
+            c.upload(sb)
+        b.set_kernel(nb.KERNEL_BVH8)
+        b.set_traversal(**a.traversal())
+        assert b.traversal() == a.traversal()
+        # changed in a field, it is an ordinary configuration
+        for change in (dict(width=4, persistent=2, short_stack=16), dict(persistent=1), dict(min_blocks=10), dict(block=64)):
+            b.set_traversal(**dict(a.traversal(), **change))
+            assert b.traversal() == dict(a.traversal(), regroup=1, **change)
+        # and so is the per-thread binary walk by its own numbers
+        b.set_traversal(**dict(a.traversal(), regroup=1))
+        assert b.traversal()["regroup"] == 1 and a.traversal()["regroup"] != 1
+        b.set_kernel(nb.KERNEL_AUTO)
+        assert b.traversal() == a.traversal()
+    finally:
+        a.close()
+        b.close()
