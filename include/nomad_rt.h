@@ -196,7 +196,8 @@ typedef struct nomad_tune_entry {
   float ms;               /* best of `repeats` timings; negative when not run                  */
   uint32_t mismatches;    /* sample rays whose hit differs from the binary per-thread kernel's */
 } nomad_tune_entry;
-/* Sweeps the six NOMAD_KERNEL_* variants, each also with min_blocks 10, 12 and 16, the hybrid
+/* Sweeps the six NOMAD_KERNEL_* variants, each also with min_blocks 10, 12 and 16 where it has those
+ * builds (see min_blocks), the hybrid
  * packet kernel at widths 2, 4, 8, and, for the regrouping kernel, width {2,4,8} x short
  * stack {0 (local), 8, 16, 32} x regroup threshold {1, 16, 24, 32} x postponed leaves {0, 1} x
  * staged top levels {0, up to 8 KB} x block {128, 256} on n sample rays, checks every

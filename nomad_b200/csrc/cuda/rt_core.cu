@@ -739,6 +739,8 @@ static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n, bool que
   return (coop_pays(ctx, n, queue) || ctx->trav.persistent != 0) && coop_traversal(ctx, &c) ? c : ctx->trav;
 }
 
+bool nomad_coop_pays(const nomad_ctx *ctx, uint64_t n) { return coop_pays(ctx, n, false); }
+
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,
                                cudaStream_t st) {

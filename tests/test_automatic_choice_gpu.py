@@ -54,3 +54,24 @@ def test_unchosen_configuration_goes_with_the_dict(nb, small_city):
     finally:
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("leaves", ["several records", "one record"])
+def test_sweep_times_no_build_twice(nb, small_city, leaves):
+    """The cooperative walk has one build, so the sweep lists min_blocks for it only where the scene's leaves hold
+    one record, which the lane-by-lane walk serves."""
+    sb = small_city[1]
+    if leaves == "one record":
+        geom = np.zeros((64, 15), np.float32)
+        geom[:, :9] = np.random.default_rng(1).uniform(-5, 5, (64, 9))
+        sb = nb.SceneBVH(nb.HostScene(np.ones(64, np.int32), geom, np.full((64, 20), 0.5, np.float32), np.arange(64),
+                                      np.ones(64, np.uint32)))
+    ctx = nb.Context(0)
+    try:
+        ctx.upload(sb)
+        res = ctx.autotune_sweep(raysets.aimed_rays(sb, 6000, 1), repeats=1)
+        bounded = sorted(name for name, cfg, ms, bad in res["entries"] if cfg["persistent"] == 1 and cfg["min_blocks"])
+        assert len(bounded) == (9 if leaves == "one record" else 0)
+        assert all(bad == 0 for _, _, ms, bad in res["entries"] if ms >= 0)
+    finally:
+        ctx.close()
