@@ -1067,24 +1067,25 @@ extern "C" nomad_status nomad_mlp_train(nomad_ctx *ctx, const float *features, c
   NOMAD_CUDA(ctx, cudaMemcpyAsync(S.T.p, targets, n * 4, cudaMemcpyHostToDevice, s));
   // Each epoch's permutation goes up on a copy stream into one of two buffers, so the host shuffles
   // and sends the next one while the steps of this one run. used[k]: the steps that read buffer k;
-  // sent: the copy the next steps wait for.
+  // sent[k]: the copy into it, which the next steps wait for, and the host before it writes that copy's
+  // source again.
   struct Events {
-    cudaEvent_t used[2] = {nullptr, nullptr}, sent = nullptr;
+    cudaEvent_t used[2] = {nullptr, nullptr}, sent[2] = {nullptr, nullptr};
     cudaStream_t copy = nullptr, compute = nullptr;
     ~Events() {  // also after an error: nothing of this call may still be in flight
       cudaStreamSynchronize(copy);
       cudaStreamSynchronize(compute);
-      for (cudaEvent_t e : {used[0], used[1], sent})
+      for (cudaEvent_t e : {used[0], used[1], sent[0], sent[1]})
         if (e) cudaEventDestroy(e);
     }
   };
   std::mt19937_64 rng(seed ^ 0x5EEDull);
-  std::vector<uint32_t> perm(n);
+  std::vector<uint32_t> perm(n), source[2];
   std::iota(perm.begin(), perm.end(), 0u);
   Events ev;
   ev.copy = ctx->copyStreams[0];
   ev.compute = s;
-  for (cudaEvent_t *e : {&ev.used[0], &ev.used[1], &ev.sent})
+  for (cudaEvent_t *e : {&ev.used[0], &ev.used[1], &ev.sent[0], &ev.sent[1]})
     NOMAD_CUDA(ctx, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   uint64_t cursor = n;
   int buf = 1;
@@ -1096,10 +1097,12 @@ extern "C" nomad_status nomad_mlp_train(nomad_ctx *ctx, const float *features, c
       if (!first) NOMAD_CUDA(ctx, cudaEventRecord(ev.used[buf], s));
       first = false;
       buf ^= 1;
+      NOMAD_CUDA(ctx, cudaEventSynchronize(ev.sent[buf]));  // at once if nothing was sent from it yet
+      source[buf] = perm;
       NOMAD_CUDA(ctx, cudaStreamWaitEvent(ev.copy, ev.used[buf], 0));
-      NOMAD_CUDA(ctx, cudaMemcpyAsync(S.perm[buf].p, perm.data(), n * 4, cudaMemcpyHostToDevice, ev.copy));
-      NOMAD_CUDA(ctx, cudaEventRecord(ev.sent, ev.copy));
-      NOMAD_CUDA(ctx, cudaStreamWaitEvent(s, ev.sent, 0));
+      NOMAD_CUDA(ctx, cudaMemcpyAsync(S.perm[buf].p, source[buf].data(), n * 4, cudaMemcpyHostToDevice, ev.copy));
+      NOMAD_CUDA(ctx, cudaEventRecord(ev.sent[buf], ev.copy));
+      NOMAD_CUDA(ctx, cudaStreamWaitEvent(s, ev.sent[buf], 0));
       cursor = 0;
     }
     TrainBufs tb;
