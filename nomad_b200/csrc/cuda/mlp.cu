@@ -725,6 +725,7 @@ __global__ void __launch_bounds__(128) k_loss(const float *__restrict__ se, int 
 
 struct MlpState {
   bool ready = false;
+  bool smemSet = false;  // the kernels opted in to their shared memory on this context's device
   DeviceBuf P, Wc, W2t, M, V, G;
   DeviceBuf X, T, perm[2], ximg, h1img, z2img, z1img, g1c, g2c, g3c, dy, se, mask, part1, part2, loss;
   DeviceBuf inX, inY;
@@ -751,8 +752,7 @@ nomad_status ensure(nomad_ctx *ctx, MlpState &S) {
   NOMAD_CUDA(ctx, S.M.reserve(kParams * 4));
   NOMAD_CUDA(ctx, S.V.reserve(kParams * 4));
   NOMAD_CUDA(ctx, S.G.reserve(kParams * 4));
-  static bool attr = false;
-  if (!attr) {
+  if (!S.smemSet) {
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_mlp_forward_tc<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kTcSmem));
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_mlp_forward_tc<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -761,7 +761,7 @@ nomad_status ensure(nomad_ctx *ctx, MlpState &S) {
                                          (int)kTcSmemTrain));
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_train_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHiddenSmem));
     NOMAD_CUDA(ctx, cudaFuncSetAttribute(k_train_input, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInputSmem));
-    attr = true;
+    S.smemSet = true;
   }
   return NOMAD_OK;
 }
