@@ -20,6 +20,7 @@
 #include <random>
 #include <vector>
 
+#include "bulk_ring.h"
 #include "residency_features.cuh"
 #include "rt_context.h"
 
@@ -563,10 +564,12 @@ __device__ __forceinline__ void ordered_sums(unsigned char *smem, int n, int c0,
   __syncthreads();
   const int tiles = (n + 127) / 128;
   bool ok = true;
+  using Ring = BulkRing<kSumRing>;
   if (warp == 1 && lane == 0) {
-    for (int t = 0; t < tiles; ++t) {
-      const int s = t % kSumRing;
-      if (t >= kSumRing && !tc_wait(bars + 8 * (kSumRing + s), (t / kSumRing - 1) & 1)) {
+    int issued = 0;
+    for (; issued < tiles; ++issued) {
+      const int t = issued, s = Ring::stage(t);
+      if (t >= kSumRing && !tc_wait(bars + 8 * (kSumRing + s), Ring::parity(t - kSumRing))) {
         ok = false;
         break;
       }
@@ -575,6 +578,8 @@ __device__ __forceinline__ void ordered_sums(unsigned char *smem, int n, int c0,
       bulk_load(base + s * kSumStage, col + (PLAIN ? (size_t)t * 128 : (size_t)t * (128 * kHid) + c0 * 128), bytes,
                 bars + 8 * s);
     }
+    // every copy has landed before the block ends, also when a wait of either warp ran out
+    for (int t = Ring::first_open(issued); t < issued; ++t) ok = tc_wait(bars + 8 * Ring::stage(t), Ring::parity(t)) && ok;
   } else if (warp == 0) {
     // chunks of 32 rows, the next one loading while one is added
     float sum = 0.0f;
@@ -608,7 +613,7 @@ __device__ __forceinline__ void ordered_sums(unsigned char *smem, int n, int c0,
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 8 * (kSumRing + (i >> 2) % kSumRing))
                          : "memory");
           const int t = next >> 2;
-          ok = __all_sync(0xffffffffu, tc_wait(bars + 8 * (t % kSumRing), (t / kSumRing) & 1));
+          ok = __all_sync(0xffffffffu, tc_wait(bars + 8 * Ring::stage(t), Ring::parity(t)));
         }
       } else {
         next = i;  // nothing follows: what is loaded is not used
@@ -617,11 +622,7 @@ __device__ __forceinline__ void ordered_sums(unsigned char *smem, int n, int c0,
     }
     if (!PLAIN || lane == 0) out[lane] = sum;
   }
-  if (!ok && lane == 0) {
-    // a wait that ran out: let the copies in flight land before the block ends
-    for (int s = 0; s < kSumRing; ++s) tc_wait(bars + 8 * s, 0);
-    atomicOr(status, kStatusWaitExpired);
-  }
+  if (!ok && lane == 0) atomicOr(status, kStatusWaitExpired);
   __syncthreads();
 }
 
