@@ -26,7 +26,8 @@
 // loads; they share a launch, their blocks alternating, so one hides the other. Flags are bits, and
 // a scan is a launch that writes them with their tiles' sums and one that adds up the sums before
 // its tile. City of 2.48M triangles at 40 % of objects:
-// 145 us (343 MB copied: 64 us at the copy rate); 205 us as 14 launches one after the other.
+// 142 us (418 MB in all: 64 us at the copy rate, 53 for the 343 MB that are copied); 209 us as 14 launches
+// one after the other.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -299,8 +300,8 @@ __device__ __forceinline__ bool node_emitted(const float4 *__restrict__ bvh, uin
 }
 
 // Emitted bits of the nodes (a thread a node, a sum per block) and the primitive copy, in alternating
-// blocks. The copy's blocks stay until it is done and take 6 of the 8 an SM holds (145 us per
-// compaction of the city; 4 of 8: 161, 5: 150, all 8: 168); the node blocks pass through the others.
+// blocks. The copy's blocks stay until it is done and take 6 of the 8 an SM holds (4 of 8: 11 % slower per
+// compaction of the city, 5: 3 %, all 8: 16 %); the node blocks pass through the others.
 __global__ void __launch_bounds__(kT, 8) k_copy_nodes(const uint32_t *__restrict__ remap, const uint32_t *__restrict__ cpos,
                                                    uint32_t n, const float4 *__restrict__ prims,
                                                    const float4 *__restrict__ mats, float4 *__restrict__ oPrims,

@@ -12,7 +12,8 @@
 //   finalize: average the samples of each pixel (clamped to [0,1] per sample and per pixel when
 //             NOMAD_VIEW_CLAMP, like pathTraceKernel)
 //
-// Queue appends are warp-aggregated (ballot + one atomic per warp). Every path owns fixed slots
+// Queue appends are aggregated: shading appends to both of its queues by the block, the reference mode's
+// candidates leave each warp 32 at a time, its reuse rays by the warp. Every path owns fixed slots
 // (throughput, radiance), so the order of a queue does not change any result, and the
 // contributions of a path are added in the reference's order: emission, then direct light, per
 // bounce. Random numbers come from Philox4x32-10 with key (seed_lo, seed_hi + frame) and counter
@@ -31,8 +32,8 @@ using namespace nomad_pt;
 namespace {
 
 constexpr int kPtBlock = 256;
-// Resident blocks per SM the ReSTIR candidate, spatial and reference-mode kernels are compiled
-// for (a register cap): 4 was measured faster than 3, 5 and the uncapped build, same images.
+// Resident blocks per SM the ReSTIR spatial and reference-mode kernels are compiled for (a register
+// cap): 4 was measured faster than 3, 5 and the uncapped build, same images.
 #ifndef NOMAD_PT_MINB
 #define NOMAD_PT_MINB 4
 #endif
@@ -424,7 +425,6 @@ __device__ __forceinline__ V3 scatter(V3 inDir, V3 normal, bool frontFace, const
   return m.transmission / prob;
 }
 
-// sampleLightPoint (PathTracing.h:582-643).
 // selectLightOffset (PathTracing.h:219-235).
 __device__ __forceinline__ uint32_t select_light(float xi, const Lights &L, uint32_t count, float total) {
   float target = xi * total;

@@ -810,8 +810,8 @@ nomad_status trace_host(nomad_ctx *ctx, Op op, const nomad_ray *rays, uint64_t n
   // 25 us of host and copy-engine time, against 150 us of upload (921,600 rays: 795 us; at least
   // 2^19: 890, 2^17: 843). The last chunk's traversal and
   // download run after every upload has landed, so a batch of more than two chunks ends with
-  // halving ones (1/2, 1/4, 1/8, 1/8 of a chunk): the part of the batch that no upload overlaps
-  // shrinks to an eighth of a chunk.
+  // halving ones, down to an eighth of a chunk or 2^16 rays (1/2, 1/4, 1/4 of the smallest chunk, 1/2, 1/4,
+  // 1/8, 1/8 of one twice as large): the part of the batch that no upload overlaps shrinks to the last one.
   const uint64_t chunk = std::max<uint64_t>(1 << 18, (n + 15) / 16);
   std::vector<uint64_t> parts;
   {
