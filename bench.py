@@ -564,6 +564,30 @@ def ingest_leg(nb):
     return out
 
 
+LINE_LIMIT = 16_000  # bytes: readers of the line take at most 32 KB of it
+
+
+def brief(x, depth):
+    """x without what lies more than `depth` levels of dicts below it, and without lists of lists or dicts."""
+    if isinstance(x, dict):
+        kept = {k: brief(v, depth - 1) for k, v in x.items() if depth > 0}
+        return {k: v for k, v in kept.items() if v is not None}
+    if isinstance(x, (list, tuple)):
+        return list(x) if len(x) <= 8 and not any(isinstance(v, (dict, list, tuple)) for v in x) else None
+    return x
+
+
+def fit_line(line, extras):
+    """The JSON line with the legs' results (`extras`), cut to the levels that fit LINE_LIMIT; the legs log them
+    whole. The line's own keys all stay, but for the autotuner's lists where even they are too long."""
+    for depth in (None, 4, 3, 2, 1, 0):
+        legs = extras if depth is None else {k: brief(v, depth) for k, v in extras.items()}
+        text = json.dumps({**line, **legs})
+        if len(text) <= LINE_LIMIT:
+            return text
+    return json.dumps({**line, "autotune": brief(line.get("autotune"), 1)})
+
+
 def select_kernel(ctx, kernel, min_blocks=0):
     """Fixes the traversal to a NOMAD_KERNEL_* variant, optionally with a min_blocks bound."""
     import nomad_b200 as nb
@@ -922,8 +946,7 @@ def main():
                 f"_mb{args.min_blocks}" if args.min_blocks else ""),
             "autotune": tune,
         }
-        line.update(extras)
-        print(json.dumps(line), flush=True)
+        print(fit_line(line, extras), flush=True)
     ctx.close()
     if world > 1:
         dist.destroy_process_group()
