@@ -389,17 +389,9 @@ extern "C" nomad_status nomad_scene_upload(nomad_ctx *ctx, const float *bvh, uin
   S.rootRef = L.rootRef;
   S.tlasPairs = L.tlasPairCount;
   S.triCount = (int32_t)primCount;
-  {  // what the choice of a persistent walk depends on
-    uint32_t leaves = 0, tris = 0;
-    for (uint32_t k = 0; k < primCount; ++k) {
-      int32_t meta;
-      std::memcpy(&meta, &L.tris[12ull * k + 11], 4);
-      leaves += (meta & kLastInLeaf) != 0;
-      tris += (meta & 0xff) == 1;
-    }
-    ctx->leafRecords = leaves ? (float)primCount / (float)leaves : 0.0f;
-    ctx->mostlyTris = 2ull * tris >= primCount;
-  }
+  // what the choice of a persistent walk depends on
+  ctx->leafRecords = L.leafCount ? (float)primCount / (float)L.leafCount : 0.0f;
+  ctx->mostlyTris = 2ull * L.triangleCount >= primCount;
   S.status = static_cast<uint32_t *>(ctx->status.p);
   ctx->primCount = primCount;
   ctx->objectCount = objectCount;

@@ -227,6 +227,7 @@ bool build_traversal_layout(const float *bvh, uint32_t bvhCount, const float *tl
 
   // Leaf-ordered triangle records, with the leaf-closing flag.
   out.tris.assign(12ull * primCount, 0.0f);
+  out.leafCount = out.triangleCount = 0;
   std::vector<uint8_t> closes(primCount, 0);
   for (uint32_t i = 0; i < bvhCount; ++i) {
     N2 n = bn(i);
@@ -250,6 +251,8 @@ bool build_traversal_layout(const float *bvh, uint32_t bvhCount, const float *tl
     t[4] = b.x; t[5] = b.y; t[6] = b.z; t[7] = int_bits_as_float(out.primObject[p]);
     t[8] = c.x; t[9] = c.y; t[10] = c.z;
     t[11] = int_bits_as_float(type | (closes[k] ? kLastInLeaf : 0));
+    out.leafCount += closes[k];
+    out.triangleCount += type == 1;
   }
   // Leaves must tile [0, primCount) with no gaps so every chain of records ends at a flag.
   for (uint32_t o = 0; o < objectCount; ++o) {
