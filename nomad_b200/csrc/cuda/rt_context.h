@@ -255,7 +255,7 @@ nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, boo
                                  const uint32_t *lenDev, unsigned long long *cursor, int32_t *hits5,
                                  uint8_t *occ, uint32_t *counts, cudaStream_t st);
 // Whether persistent = 1 walks a batch of n rays of this scene with cooperative leaf tests.
-bool nomad_coop_pays(const nomad_ctx *ctx, uint64_t n);
+bool nomad_coop_pays(const nomad_ctx *ctx, uint32_t width, uint64_t n);
 // The same trace with the context's configuration, or the library's choice where the caller made none.
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,

@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <new>
 #include <string>
@@ -604,11 +605,13 @@ constexpr int kStackW4 = 64, kStackW8 = 96;
 // the time). With two records a leaf the tests gain as much as they lose. In batches of up
 // to a ray for each of 28 warps per SM the equal shares of the cooperative kernel decide (1,000 rays: 0.7 to
 // 1.0 of the time), in a frame's queues, which shrink from bounce to bounce, up to 32 rays (57,600 paths
-// of two bounces: 467 us with the tests, 519 without). What remains slower with the tests are coherent
+// of two bounces: 467 us with the tests, 519 without); not over 2-wide nodes, where a lane reaches a leaf after more
+// steps (1,000 rays 83 us with the tests, 75 without). What remains slower with the tests are coherent
 // batches of about a million rays into scenes of less than a few hundred primitives (250 triangles: 1.1 to
 // 1.25; incoherent ones 0.5).
-bool coop_pays(const nomad_ctx *ctx, uint64_t n, bool queue) {
-  return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) || n <= ctx->smCount * (queue ? 896ull : 28ull);
+bool coop_pays(const nomad_ctx *ctx, uint32_t width, uint64_t n, bool queue) {
+  return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) ||
+         (width != 2 && n <= ctx->smCount * (queue ? 896ull : 28ull));
 }
 
 template <int W, int STACK, bool ANY, Walk WALK, int MINB>
@@ -677,7 +680,7 @@ nomad_status launch_walk(nomad_ctx *ctx, const nomad_traversal &c, const WideSce
                          uint32_t *counts, cudaStream_t st) {
   if (c.persistent == 0)
     return launch_minb<W, STACK, ANY, Walk::PerThread>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
-  if (cursor && !coop_pays(ctx, n, lenDev != nullptr))
+  if (cursor && !coop_pays(ctx, c.width, n, lenDev != nullptr))
     return launch_minb<W, STACK, ANY, Walk::PerLane>(ctx, c.min_blocks, WS, rays, n, lenDev, cursor, hits5, occ, counts, st);
   // one build each, at the occupancy that was measured best
   return ctx->mostlyTris
@@ -716,22 +719,27 @@ nomad_status nomad_trace_variant(nomad_ctx *ctx, const nomad_traversal &cfg, boo
 // The configuration that serves a context whose caller has not chosen one: the cooperative kernel
 // over 4-wide nodes (2.2 times the per-thread binary walk's speed on a 58k-ray frame, 1.3 to 1.7 on
 // millions of rays), or another width where that layout is not on the device or would need a
-// deeper stack. Where it does not pay, the per-thread binary walk, unless only a wider layout is on
-// the device (paging).
-static bool coop_traversal(const nomad_ctx *ctx, nomad_traversal *c) {
-  for (uint32_t k : {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}) {
+// deeper stack. Where it does not pay, the per-thread walk over binary nodes, or over those that are on the
+// device (paging).
+static bool first_ok(const nomad_ctx *ctx, std::initializer_list<uint32_t> kernels, nomad_traversal *c) {
+  for (uint32_t k : kernels) {
     *c = nomad_kernel_config(k);
     if (nomad_traversal_ok(ctx, *c, nullptr)) return true;
   }
   return false;
 }
 
-static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n, bool queue) {
-  nomad_traversal c;
-  return (coop_pays(ctx, n, queue) || ctx->trav.persistent != 0) && coop_traversal(ctx, &c) ? c : ctx->trav;
+static bool coop_traversal(const nomad_ctx *ctx, nomad_traversal *c) {
+  return first_ok(ctx, {NOMAD_KERNEL_BVH4_PERSIST, NOMAD_KERNEL_BVH2_PERSIST, NOMAD_KERNEL_BVH8_PERSIST}, c);
 }
 
-bool nomad_coop_pays(const nomad_ctx *ctx, uint64_t n) { return coop_pays(ctx, n, false); }
+static nomad_traversal auto_traversal(const nomad_ctx *ctx, uint64_t n, bool queue) {
+  nomad_traversal c;
+  if (coop_traversal(ctx, &c) && coop_pays(ctx, c.width, n, queue)) return c;
+  return first_ok(ctx, {NOMAD_KERNEL_BVH2, NOMAD_KERNEL_BVH4, NOMAD_KERNEL_BVH8}, &c) ? c : ctx->trav;
+}
+
+bool nomad_coop_pays(const nomad_ctx *ctx, uint32_t width, uint64_t n) { return coop_pays(ctx, width, n, false); }
 
 nomad_status nomad_trace_queue(nomad_ctx *ctx, bool any, const float4 *rays, uint64_t n, const uint32_t *lenDev,
                                unsigned long long *cursor, int32_t *hits5, uint8_t *occ, uint32_t *counts,

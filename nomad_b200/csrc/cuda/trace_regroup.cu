@@ -647,7 +647,7 @@ extern "C" nomad_status nomad_autotune_sweep(nomad_ctx *ctx, const nomad_ray *ra
   for (uint32_t k = NOMAD_KERNEL_BVH2; k < NOMAD_KERNEL_COUNT; ++k)
     for (uint32_t mb : {10u, 12u, 16u}) {
       nomad_traversal c = nomad_kernel_config(k);
-      if (c.persistent == 1 && nomad_coop_pays(ctx, n)) break;  // one build, measured above
+      if (c.persistent == 1 && nomad_coop_pays(ctx, c.width, n)) break;  // one build, measured above
       c.min_blocks = mb;
       grid.push_back(c);
     }

@@ -82,7 +82,32 @@ def test_frames(nb, kind, prims, objects, w, h, spp):
         ctx.close()
 
 
-def _times(nb, sb, kernels):
+@pytest.mark.parametrize("width", [2, 4, 8])
+def test_paged_one_record_leaves(nb, width):
+    """An untuned context whose only layout is a paged one, batches and frames on both sides of the lines."""
+    sb = _scene(nb, 1, 300, 300)
+    rays = np.concatenate([raysets.aimed_rays(sb, 4144, 1), raysets.random_rays(sb, 2000, 2)])
+    v = nb.view_pinhole((0, 10, -60), (0, 0, 0), width=383, height=401, spp=1, max_depth=3, seed=3)
+    out = []
+    for paged in (False, True):
+        ctx = nb.Context(0)
+        try:
+            ctx.upload(sb)
+            if paged:
+                ctx.paging_enable(1 << 40, width=width, max_onloads=sb.object_count)
+                for _ in range(4):
+                    ctx.paging_update()
+                    ctx.paging_wait()
+                assert ctx.paging_stats()["resident"] == sb.object_count
+            out.append([_bits(ctx.trace_closest(rays[:n])) for n in (1, 4144, 4145, 6144)] +
+                       [ctx.trace_any(rays), ctx.render(v)[0].view(np.int32), ctx.render(v[:1])[0].view(np.int32)])
+            assert ctx.status() == 0
+        finally:
+            ctx.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def _times(nb, sb, kernels, paged=0):
     """Milliseconds of a million coherent closest hits with each kernel, the best of twelve."""
     import torch
 
@@ -96,6 +121,11 @@ def _times(nb, sb, kernels):
     ctx = nb.Context(0)
     try:
         ctx.upload(sb)
+        if paged:
+            ctx.paging_enable(1 << 40, width=paged, max_onloads=sb.object_count)
+            for _ in range(4):
+                ctx.paging_update()
+                ctx.paging_wait()
         best = []
         for kernel in kernels:
             ctx.set_kernel(kernel)
@@ -117,6 +147,12 @@ def test_untuned_on_one_record_leaves(nb):
     """A million rays into 8,192 objects of one triangle: the untuned context takes at most 1.1 times as long as
     the per-thread binary walk (1.2 to 1.45 with cooperative leaf tests)."""
     auto, walk = _times(nb, _scene(nb, 1, 8192, 8192), (0, 1))
+    assert auto <= 1.1 * walk, (auto, walk)
+
+
+def test_paged_untuned_on_one_record_leaves(nb):
+    """The same with a paged 4-wide layout, against its per-thread walk."""
+    auto, walk = _times(nb, _scene(nb, 1, 8192, 8192), (0, 3), paged=4)
     assert auto <= 1.1 * walk, (auto, walk)
 
 
