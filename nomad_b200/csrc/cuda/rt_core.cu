@@ -608,7 +608,7 @@ constexpr int kStackW4 = 64, kStackW8 = 96;
 // of two bounces: 467 us with the tests, 519 without); not over 2-wide nodes, where a lane reaches a leaf after more
 // steps (1,000 rays 83 us with the tests, 75 without). What remains slower with the tests are coherent
 // batches of about a million rays into scenes of less than a few hundred primitives (250 triangles: 1.1 to
-// 1.25; incoherent ones 0.5).
+// 1.25, incoherent ones 0.5; 250 spheres: 1.2 to 1.4 and 0.8).
 bool coop_pays(const nomad_ctx *ctx, uint32_t width, uint64_t n, bool queue) {
   return (ctx->leafRecords >= 1.5f && ctx->primCount >= 16) ||
          (width != 2 && n <= ctx->smCount * (queue ? 896ull : 28ull));
