@@ -32,8 +32,8 @@ from . import native as nat
 
 HIST_FEATURES = list(range(3, 12)) + [19, 20]
 HYSTERESIS = 0.5  # resident_key_bonus of the hysteresis rows
-# the traversal of every context of the workload: 4-wide nodes, persistent warps, 10 blocks per SM
-# (the bench city's autotuned choice)
+# the traversal of every context of the workload: 4-wide nodes, persistent warps (the bench city's
+# autotuned choice); min_blocks would apply to the lane-by-lane walk, which this city does not take
 TRAVERSAL = dict(width=4, persistent=1, short_stack=0, regroup=1, staged_nodes=0, block=128, postpone_leaves=0,
                  min_blocks=10)
 VALIDATION_PATH = 2  # camera path on which the paged configuration is chosen (evaluation: path 1)
